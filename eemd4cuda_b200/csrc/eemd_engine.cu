@@ -27,6 +27,7 @@
 #include <cstdio>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 namespace cg = cooperative_groups;
@@ -53,18 +54,6 @@ __device__ __forceinline__ double rnd(double v) { return (double)(T)v; }
 __device__ __forceinline__ float fmat(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fmat(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-// knot sample index kept in a storage-type record plane as an integer bit pattern
-template <typename T>
-__device__ __forceinline__ T tbits(int t) {
-    if constexpr (sizeof(T) == 4) return __int_as_float(t);
-    else return __longlong_as_double((long long)t);
-}
-template <typename T>
-__device__ __forceinline__ int tint(T v) {
-    if constexpr (sizeof(T) == 4) return __float_as_int(v);
-    else return (int)__double_as_longlong(v);
-}
-
 // 1/x: hardware approximation refined by one Newton step on f(y) = 1/y - x,
 // y <- y + y(1 - xy); relative error about 2^-50 or better.
 __device__ __forceinline__ double fast_rcp(double x) {
@@ -84,14 +73,26 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+// 256-bit global accesses (sm_100): a lane's run of samples, 32-byte aligned.
+// The loads leave L1 to the interval records (samples are read once per step).
+__device__ __forceinline__ void ld256(const float* p, float (&v)[8]) {
+    asm volatile("ld.global.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
 }
-template <typename T>
-__device__ __forceinline__ void cp_async_el(T* smem, const T* gmem) {
-    if (sizeof(T) == 8) cp_async8(smem, gmem);
-    else cp_async4(smem, gmem);
+__device__ __forceinline__ void ld256(const double* p, double (&v)[4]) {
+    asm volatile("ld.global.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];\n"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                 : "l"(p));
+}
+__device__ __forceinline__ void st256(float* p, const float (&v)[8]) {
+    asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};\n" ::"f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void st256(double* p, const double (&v)[4]) {
+    asm volatile("st.global.v4.f64 [%4], {%0, %1, %2, %3};\n" ::"d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]), "l"(p)
+                 : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -252,26 +253,15 @@ __device__ __forceinline__ void task_error(const Ctx& C, TaskSm& S, int code) {
     } while (0)
 #endif
 
-// Per-warp sweep geometry for storage type T.  A warp tile is WT = 32*RUN
-// samples; each warp owns, in dynamic shared memory, two tile buffers per
-// stream (h, residual) and two sets of run records.  Interval records are
-// RS storage-type elements (32 or 48 bytes).
+// Sweep geometry for storage type T.  A warp tile is WT = 32*RUN samples: each
+// lane owns a run of RUN consecutive samples, 32 bytes, which one 256-bit load
+// brings into registers (and one 256-bit store writes back).
 template <typename T>
 struct Geo {
     static constexpr int RUN = sizeof(T) == 4 ? 8 : 4;  // consecutive samples per lane
     static constexpr int WT = 32 * RUN;                 // samples per warp tile
-    static constexpr int TB = WT + 4;                   // tile buffer elements (16-byte phase)
-    static constexpr int RS = sizeof(T) == 4 ? 8 : 6;   // interval record stride
-    static constexpr int NBUF = TILE_BUFS;               // tiles in flight per warp (ring)
-    static constexpr size_t TB_BYTES = (size_t)NBUF * 2 * TB * sizeof(T);  // [buf][stream][TB]
-    static constexpr size_t RI_BYTES = (size_t)NBUF * 32 * 16;          // [buf][lane]
-    static constexpr int KCAP = WT / 2 + 4;                              // knots of one kind in a tile
-    static constexpr size_t KN_BYTES = (size_t)2 * KCAP * (4 + sizeof(T));  // [kind][KCAP] index, value
-    static constexpr size_t WARP_BYTES = TB_BYTES + RI_BYTES + KN_BYTES;
-    static_assert(TB_BYTES % 16 == 0 && (RS * sizeof(T)) % 16 == 0 && KN_BYTES % 16 == 0,
-                  "16-byte aligned layouts");
+    static constexpr int RS = sizeof(T) == 4 ? 8 : 6;   // workspace elements per interval record
 };
-
 
 __host__ __device__ inline int stage_pad(int k) { return k + (k >> 4); }
 
@@ -299,19 +289,17 @@ constexpr int WSCAP_FAST = FAST_ROWS + FAST_SMAX + 3;
 __host__ __device__ constexpr int stage_cap(bool exact) { return exact ? WSCAP : WSCAP_FAST; }
 
 // per-warp solve area: slopes (double), knot times (int), knot values
-// (storage type), and in fast mode the forward (c, d) of a pass's rows.  It
-// overlays the sweep's area; keeping it no larger leaves the L1 share of the
-// SM's on-chip memory (used by the sweep's record loads) unchanged.
+// (storage type), and in fast mode the forward (c, d) of a pass's rows.  What
+// it leaves of the SM's on-chip memory is L1, which the sweep's record
+// gathers live in.
 __host__ __device__ inline size_t wsolve_bytes(size_t bt, bool exact) {
     const size_t sp = (size_t)stage_pad(stage_cap(exact));
     return align16(sp * 8) + align16(sp * 4) + align16(sp * bt) + (exact ? 0 : (size_t)FAST_ROWS * 16);
 }
 
-// dynamic shared memory of k_emd: the sweep's and the solve's per-warp areas overlay
+// dynamic shared memory of k_emd: the solve's per-warp areas (the sweep works in registers)
 __host__ __device__ inline size_t smem_bytes(int bt, bool exact, int nw) {
-    const size_t sweep = nw * (bt == 8 ? Geo<double>::WARP_BYTES : Geo<float>::WARP_BYTES);
-    const size_t solve = nw * wsolve_bytes((size_t)bt, exact);
-    return sweep > solve ? sweep : solve;
+    return nw * wsolve_bytes((size_t)bt, exact);
 }
 
 // ---------------------------------------------------------------------------
@@ -319,12 +307,12 @@ __host__ __device__ inline size_t smem_bytes(int bt, bool exact, int nw) {
 // position i - pref[r] of that segment's list
 // ---------------------------------------------------------------------------
 struct Slot {
-    int32_t* kt;   // knot lists (segmented)
-    void* ky;
-    void* M;       // interval records, mirror space: [2 env][5][kcap] storage type
+    int32_t* kt;   // knot lists (segmented): float32 storage pairs of (index, value),
+    void* ky;      //   float64 storage indices here and values in ky
+    void* M;       // interval records, mirror space (struct Rec)
     void* w1;      // scratch h buffer of the running task (storage type)
     void* r1;      // second residual buffer of the running task (storage type)
-    int4* ri;      // run records [2 parity][runs]: first knot of each kind, knot masks
+    uint32_t* ri;  // run records [2 parity][runs] (run_record)
 };
 
 __device__ __forceinline__ int64_t knot_index(const Ctx& C, int par, int env, int seg, int i) {
@@ -348,12 +336,35 @@ __device__ __forceinline__ int64_t real_off(const Ctx& C, const TaskSm& S, int e
     return knot_index(C, S.kpar, env, r, i - pr[r]);
 }
 
+// knot at element offset o of the lists: float32 storage keeps (index, value)
+// pairs, so a knot is one 8-byte access; float64 storage two arrays
+template <typename T>
+__device__ __forceinline__ void get_knot(const Slot& sl, int64_t o, int& t, T& y) {
+    if constexpr (sizeof(T) == 4) {
+        const int2 k = __ldcg(reinterpret_cast<const int2*>(sl.kt) + o);
+        t = k.x;
+        y = __int_as_float(k.y);
+    } else {
+        t = __ldcg(sl.kt + o);
+        y = __ldcg(static_cast<const T*>(sl.ky) + o);
+    }
+}
+template <typename T>
+__device__ __forceinline__ void put_knot(const Slot& sl, int64_t o, int t, T y) {
+    if constexpr (sizeof(T) == 4) {
+        reinterpret_cast<int2*>(sl.kt)[o] = make_int2(t, __float_as_int(y));
+    } else {
+        sl.kt[o] = t;
+        static_cast<T*>(sl.ky)[o] = y;
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ void real_knot(const Ctx& C, const Slot& sl, const TaskSm& S, int env, int i,
                                           int& t, double& y) {
-    const int64_t o = real_off(C, S, env, i);
-    t = __ldcg(sl.kt + o);
-    y = (double)__ldcg(static_cast<const T*>(sl.ky) + o);
+    T v;
+    get_knot<T>(sl, real_off(C, S, env, i), t, v);
+    y = (double)v;
 }
 
 // Stage the mirror-space knots rlo .. rlo+kcount-1 (lane-strided); each lane
@@ -392,8 +403,13 @@ __device__ __forceinline__ void stage_range(const Ctx& C, const Slot& sl, TaskSm
         }
 #endif
         const int64_t o = knot_index(C, S.kpar, env, r, i2 - pr[r]);
-        cp_async4(kt_s, sl.kt + o);
-        cp_async_el<T>(ky_s, static_cast<const T*>(sl.ky) + o);
+        if constexpr (sizeof(T) == 4) {
+            cp_async4(kt_s, sl.kt + 2 * o);
+            cp_async4(ky_s, sl.kt + 2 * o + 1);
+        } else {
+            cp_async4(kt_s, sl.kt + o);
+            cp_async8(ky_s, static_cast<const T*>(sl.ky) + o);
+        }
     }
 }
 
@@ -451,13 +467,28 @@ __device__ __forceinline__ Row row_of(int ta, int tb, int tc, double sa, double 
 #define SKT(k) skt[stage_slot<kExact>(k)]
 #define SSL(k) ssl[stage_slot<kExact>(k)]
 
-// Interval records of one envelope in mirror space: RS storage-type elements
-// per record: [0] t_k (integer bit pattern), [1] y_k, [2] fast: c1 / exact:
-// M_k, [3] c2, [4] c3.
+// Interval records of one envelope in mirror space: for interval k (knots k,
+// k+1) the four coefficients c[4k..4k+3] (fast: y_k, c1, c2, c3 of the
+// monomial; exact: y_k, M_k), one 16-byte (float32) or 32-byte (float64) vector
+// that the sweep gathers with one load, and apart from them the knot's sample
+// index t[k], read once per run of samples.
 template <typename T>
 struct Rec {
-    T* rc;
-    __device__ __forceinline__ T& at(int k, int e) const { return rc[(int64_t)k * Geo<T>::RS + e]; }
+    T* c;
+    int32_t* t;
+    __device__ __forceinline__ Rec(void* M, int env, int kcap) {
+        c = static_cast<T*>(M) + (int64_t)env * 4 * kcap;
+        t = reinterpret_cast<int32_t*>(static_cast<T*>(M) + (int64_t)8 * kcap) + (int64_t)env * kcap;
+    }
+    __device__ __forceinline__ void put(int k, int tk, T y, T c1, T c2, T c3) const {
+        t[k] = tk;
+        if constexpr (sizeof(T) == 4) {
+            reinterpret_cast<float4*>(c)[k] = make_float4(y, c1, c2, c3);
+        } else {
+            const T v[4] = {y, c1, c2, c3};
+            st256(c + 4 * (int64_t)k, v);
+        }
+    }
 };
 
 // exact: forward elimination from w0 (outer coupling dropped), back
@@ -491,9 +522,7 @@ __device__ void window_exact(const Ctx& C, const int* skt, const T* sky, const d
         sa = sb;
     }
     auto put = [&](int k, double Mk) {
-        R.at(k, 0) = tbits<T>(SKT(k - base));
-        R.at(k, 1) = sky[stage_slot<kExact>(k - base)];
-        R.at(k, 2) = (T)Mk;
+        R.put(k, SKT(k - base), sky[stage_slot<kExact>(k - base)], (T)Mk, (T)0, (T)0);
     };
     double xv = dp;
     if (w1 <= o1) put(w1 + 1, xv);
@@ -557,11 +586,9 @@ __device__ __forceinline__ void window_fast_back(const int* skt, const T* sky, c
     auto put = [&](int k, double Ma, double Mb) {
         const int t0 = SKT(k - base), t1 = SKT(k + 1 - base);
         const double h = (double)(t1 - t0);
-        R.at(k, 0) = tbits<T>(t0);
-        R.at(k, 1) = sky[stage_slot<kExact>(k - base)];
-        R.at(k, 2) = (T)fma(-h * (1.0 / 6.0), fma(2.0, Ma, Mb), SSL(k - base));
-        R.at(k, 3) = (T)(0.5 * Ma);
-        R.at(k, 4) = (T)((Mb - Ma) * fast_rcp(h) * (1.0 / 6.0));
+        R.put(k, t0, sky[stage_slot<kExact>(k - base)],
+              (T)fma(-h * (1.0 / 6.0), fma(2.0, Ma, Mb), SSL(k - base)), (T)(0.5 * Ma),
+              (T)((Mb - Ma) * fast_rcp(h) * (1.0 / 6.0)));
     };
     double xn = 0.0;  // x_{i+1}: zero past the natural end (M = 0) or at the truncation
     for (int i = rh; i >= o0; --i) {
@@ -597,20 +624,16 @@ __device__ void solve_task(const Ctx& C, const Slot& sl, TaskSm& S, unsigned cha
     for (int env = 0; env < 2; ++env) {
         const int p2 = S.p2[env];
         if (p2 - 2 > 0 || S.rank != 0 || tid >= p2) continue;
-        Rec<T> R;
-        R.rc = static_cast<T*>(sl.M) + (int64_t)env * C.kcap * Geo<T>::RS;
+        const Rec<T> R(sl.M, env, C.kcap);
         int tk, t1;
         double yk, y1;
         knot2<T>(C, sl, S, env, tid, tk, yk);
-        R.at(tid, 0) = tbits<T>(tk);
-        R.at(tid, 1) = (T)yk;
-        R.at(tid, 2) = (T)0;
-        R.at(tid, 3) = (T)0;
-        R.at(tid, 4) = (T)0;
+        T c1 = (T)0;
         if (!EXACT && tid + 1 < p2) {
             knot2<T>(C, sl, S, env, tid + 1, t1, y1);
-            R.at(tid, 2) = (T)((y1 - yk) / (double)(t1 - tk));
+            c1 = (T)((y1 - yk) / (double)(t1 - tk));
         }
+        R.put(tid, tk, (T)yk, c1, (T)0, (T)0);
     }
     // The windows of both envelopes form one list (envelope 0 first); CTA r
     // takes an even share of it and each warp a contiguous part of the CTA's
@@ -671,8 +694,7 @@ __device__ void solve_task(const Ctx& C, const Slot& sl, TaskSm& S, unsigned cha
         }
         __syncwarp();
         SUB(1);
-        Rec<T> R;
-        R.rc = static_cast<T*>(sl.M) + (int64_t)env * C.kcap * Geo<T>::RS;
+        const Rec<T> R(sl.M, env, C.kcap);
         const int w = w0 + lane;
         if (EXACT) {
             if (lane < nl) window_exact<T>(C, skt, sky, ssl, rlo, n, w, R, p2);
@@ -718,40 +740,32 @@ struct Iv {
     T y0, c1, c2, c3, y1, m1;  // fast: y0 + s(c1 + s(c2 + s c3)); exact: y0, M0 = c1, y1, M1
 };
 
-// loads interval record k (and k+1 in exact mode) of an envelope's record array
-template <typename T, bool EXACT>
-__device__ __forceinline__ void load_iv(Iv<T>& v, const T* R, int k) {
-    constexpr int RS = Geo<T>::RS;
-    v.k = k;
-    const T* p = R + (int64_t)k * RS;
+// the four coefficients of interval record k
+template <typename T>
+__device__ __forceinline__ void load_coef(const T* c, int k, T& y0, T& c1, T& c2, T& c3) {
     if constexpr (sizeof(T) == 4) {
-        const float4 a = *reinterpret_cast<const float4*>(p);
-        v.t0 = __float_as_int(a.x);
-        v.y0 = a.y;
-        v.c1 = a.z;
-        v.c2 = a.w;
-        v.c3 = p[4];
-        if (EXACT) {
-            const float4 c = *reinterpret_cast<const float4*>(p + RS);
-            v.t1 = __float_as_int(c.x);
-            v.y1 = c.y;
-            v.m1 = c.z;
-        }
+        const float4 a = reinterpret_cast<const float4*>(c)[k];
+        y0 = a.x;
+        c1 = a.y;
+        c2 = a.z;
+        c3 = a.w;
     } else {
-        const double2 a = *reinterpret_cast<const double2*>(p);
-        const double2 b = *reinterpret_cast<const double2*>(p + 2);
-        v.t0 = (int)__double_as_longlong(a.x);
-        v.y0 = a.y;
-        v.c1 = b.x;
-        v.c2 = b.y;
-        v.c3 = p[4];
-        if (EXACT) {
-            const double2 c = *reinterpret_cast<const double2*>(p + RS);
-            const double2 e = *reinterpret_cast<const double2*>(p + RS + 2);
-            v.t1 = (int)__double_as_longlong(c.x);
-            v.y1 = c.y;
-            v.m1 = e.x;
-        }
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];\n"
+                     : "=d"(y0), "=d"(c1), "=d"(c2), "=d"(c3)
+                     : "l"(c + 4 * (int64_t)k));
+    }
+}
+
+// loads interval record k (and k+1 in exact mode) of an envelope's records
+template <typename T, bool EXACT>
+__device__ __forceinline__ void load_iv(Iv<T>& v, const Rec<T>& R, int k) {
+    v.k = k;
+    v.t0 = R.t[k];
+    load_coef<T>(R.c, k, v.y0, v.c1, v.c2, v.c3);
+    if (EXACT) {
+        T a, b;
+        v.t1 = R.t[k + 1];
+        load_coef<T>(R.c, k + 1, v.y1, v.m1, a, b);
     }
 }
 
@@ -764,95 +778,43 @@ __device__ __forceinline__ T iv_eval(const Iv<T>& v, int t) {
     return fmat(s, fmat(s, fmat(s, v.c3, v.c2), v.c1), v.y0);
 }
 
-__device__ __forceinline__ int mirror_adj(const TaskSm& S, int env, int t) {
-    return S.mir[env] ? (S.tfirst[env] < t ? 1 : 0) + (S.tlast[env] < t ? 1 : 0) : 0;
-}
-
 // envelope value at t with `cless` real knots strictly before t: mirror-space
-// interval = searchsorted - 1 clipped (emd_ref.py:70); reloads the interval
-// record only when the interval changes
+// interval = searchsorted - 1 clipped (emd_ref.py:70), that is (knots before t)
+// + mir - 1 clipped to [0, p2 - 2] (where a sample lies outside the virtual
+// mirror knots too, the clip gives the same interval); reloads the interval
+// record only when the interval changes.  One knot: the constant y of record 0.
 template <typename T, bool EXACT>
-__device__ __forceinline__ T env_at(const Ctx& C, const TaskSm& S, Iv<T>& v, const T* R, int env, int cless, int t) {
-    if (S.P[env] < 2) return (T)S.cval[env];
-    const int idx2 = max(0, min(cless + mirror_adj(S, env, t) - 1, S.p2[env] - 2));
-    if (idx2 != v.k) load_iv<T, EXACT>(v, R, idx2);
+__device__ __forceinline__ T env_at(const TaskSm& S, Iv<T>& v, const Rec<T>& R, int env, int cless, int t) {
+    const int p2 = S.p2[env];
+    if (p2 < 2) return R.c[0];
+    const int k = max(0, min(cless + S.mir[env] - 1, p2 - 2));
+    if (k != v.k) load_iv<T, EXACT>(v, R, k);
     return iv_eval<T, EXACT>(v, t);
 }
 
-// element phase of an address within its 16-byte block
-template <typename T>
-__device__ __forceinline__ int phase16(const T* p) {
-    return (int)((reinterpret_cast<uintptr_t>(p) / sizeof(T)) & (16 / sizeof(T) - 1));
-}
-
-// One warp copies g[0 .. cnt) to the 16-byte aligned shared dst[0 .. cnt):
-// 16-byte copies when g is 16-byte aligned too, element copies otherwise.
-template <typename T>
-__device__ __forceinline__ void tile_copy(T* dst, const T* g, int cnt, int lane) {
-    constexpr int VEC = 16 / (int)sizeof(T);
-    if (phase16(g) == 0) {
-        const int nvec = cnt / VEC;
-        for (int v = lane; v < nvec; v += 32) cp_async16(dst + v * VEC, g + v * VEC);
-        for (int j = nvec * VEC + lane; j < cnt; j += 32) cp_async_el<T>(dst + j, g + j);
-    } else {
-        for (int j = lane; j < cnt; j += 32) cp_async_el<T>(dst + j, g + j);
-    }
-}
-
-// a lane's run of RUN samples from a 16-byte aligned shared tile position
+// a lane's run of RUN samples (nv of them inside the range): one 256-bit
+// access when it is whole and p's array is 32-byte aligned, element accesses
+// otherwise
 template <typename T, int RUN>
-__device__ __forceinline__ void load_run(const T* p, T (&v)[RUN]) {
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll
-        for (int i = 0; i < RUN; i += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(p + i);
-            v[i] = a.x;
-            v[i + 1] = a.y;
-            v[i + 2] = a.z;
-            v[i + 3] = a.w;
-        }
+__device__ __forceinline__ void load_run(const T* p, T (&v)[RUN], int nv, bool vec) {
+    if (vec && nv == RUN) {
+        ld256(p, v);
     } else {
 #pragma unroll
-        for (int i = 0; i < RUN; i += 2) {
-            const double2 a = *reinterpret_cast<const double2*>(p + i);
-            v[i] = a.x;
-            v[i + 1] = a.y;
-        }
+        for (int i = 0; i < RUN; ++i) v[i] = (i < nv) ? p[i] : (T)0;
     }
 }
-
-// stores a thread's run of samples: 16-byte vectors when the run is full and
-// aligned, element stores otherwise
 template <typename T, int RUN>
-__device__ __forceinline__ void store_run(T* p, const T (&v)[RUN], int nv) {
-    if (nv == RUN && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-        if constexpr (sizeof(T) == 4) {
-#pragma unroll
-            for (int i = 0; i < RUN; i += 4)
-                *reinterpret_cast<float4*>(p + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-        } else {
-#pragma unroll
-            for (int i = 0; i < RUN; i += 2) *reinterpret_cast<double2*>(p + i) = make_double2(v[i], v[i + 1]);
-        }
-        return;
-    }
-#pragma unroll
-    for (int i = 0; i < RUN; ++i)
-        if (i < nv) p[i] = v[i];
-}
-
-// a lane's run of RUN values into a 16-byte aligned shared position
-template <typename T, int RUN>
-__device__ __forceinline__ void store_run_smem(T* p, const T (&v)[RUN]) {
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll
-        for (int i = 0; i < RUN; i += 4)
-            *reinterpret_cast<float4*>(p + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+__device__ __forceinline__ void store_run(T* p, const T (&v)[RUN], int nv, bool vec) {
+    if (vec && nv == RUN) {
+        st256(p, v);
     } else {
 #pragma unroll
-        for (int i = 0; i < RUN; i += 2) *reinterpret_cast<double2*>(p + i) = make_double2(v[i], v[i + 1]);
+        for (int i = 0; i < RUN; ++i)
+            if (i < nv) p[i] = v[i];
     }
 }
+__device__ __forceinline__ bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }
 
 // value at tile position pos (lane pos/RUN, element pos%RUN), to every lane
 template <typename T, int RUN>
@@ -863,6 +825,15 @@ __device__ __forceinline__ T tile_at(const T (&v)[RUN], int pos) {
     for (int i = 1; i < RUN; ++i)
         if (e == i) x = v[i];
     return __shfl_sync(0xffffffffu, x, pos / RUN);
+}
+
+// Run record of one lane's run, 32 bits: the knots of each kind the tile holds
+// before the run (maxima in bits 0-7, minima in 8-15; a tile holds at most
+// WT / 2 = 128 of a kind) and the run's knot masks (maxima 16-23, minima
+// 24-31).  The reader of a range adds the tiles' totals up itself, so the
+// record needs no list position.
+__device__ __forceinline__ uint32_t run_record(int px, int pn, unsigned mx, unsigned mn) {
+    return (uint32_t)px | ((uint32_t)pn << 8) | (mx << 16) | (mn << 24);
 }
 
 // Pointers and flags of one sweep step.
@@ -892,16 +863,16 @@ __device__ __forceinline__ void plain_value(const Ctx& C, const TaskSm& S, const
 // next-knot value of a sample outside the warp range (t = range start - 1 or
 // range end), evaluated by one lane from global memory
 template <typename T, bool EXACT, int MODE>
-__device__ T outside_g(const Ctx& C, const TaskSm& S, const TaskDesc& d, const StepIo<T>& io, const T* R0,
-                       const T* R1, int t, int cl0, int cl1) {
+__device__ T outside_g(const Ctx& C, const TaskSm& S, const TaskDesc& d, const StepIo<T>& io, const Rec<T>& R0,
+                       const Rec<T>& R1, int t, int cl0, int cl1) {
     constexpr bool SIFTING = (MODE == TM_SIFT || MODE == TM_LAST);
     const T h = (SIFTING || (MODE == TM_TRANS && !S.imf_from_resid)) ? __ldcg(io.hsrc + t) : (T)0;
     const T r = (MODE == TM_LAST || MODE == TM_TRANS) ? __ldcg(io.rcur + t) : (T)0;
     if (SIFTING) {
         Iv<T> v0, v1;
         v0.k = v1.k = -1;
-        const T eu = env_at<T, EXACT>(C, S, v0, R0, 0, cl0, t);
-        const T el = env_at<T, EXACT>(C, S, v1, R1, 1, cl1, t);
+        const T eu = env_at<T, EXACT>(S, v0, R0, 0, cl0, t);
+        const T el = env_at<T, EXACT>(S, v1, R1, 1, cl1, t);
         const T fn = h - (T)0.5 * (eu + el);
         return (MODE == TM_LAST) ? r - fn : fn;
     }
@@ -911,17 +882,20 @@ __device__ T outside_g(const Ctx& C, const TaskSm& S, const TaskDesc& d, const S
 }
 
 // The sweep.  The CTA's segment [s0, s1) is cut into warp tiles of WT = 32*RUN
-// samples and warp w owns the contiguous tiles [w*NT/8, (w+1)*NT/8); lane u
-// of a tile owns the run of RUN samples at u*RUN.  Each warp works through
-// its range without block-wide barriers and keeps its own knot lists (one
-// knot segment per warp, so no cross-warp prefix is needed).  Per tile:
-//   - the tile's samples of each stream it reads and its run records from
-//     the previous step (per run: position of the run's first current knot
-//     of each kind in the warp's knot lists, and the run's knot masks) are
-//     already in shared memory: cp.async, issued during the previous tile;
-//   - each lane knows the interval of every sample from its run record, and
-//     loads an interval record (32 or 48 bytes) only when the interval
-//     changes; interior tiles take a path without end handling;
+// samples and warp w owns a contiguous range of them; lane u of a tile owns
+// the run of RUN samples at u*RUN.  Each warp works through its range without
+// block-wide barriers and without shared memory, and keeps its own knot lists
+// (one knot segment per warp, so no cross-warp prefix is needed).  Per tile:
+//   - the lane's run of each stream it reads and its run record from the
+//     previous step were loaded into registers during the previous tile (one
+//     256-bit load per stream);
+//   - the run record gives each lane the interval of its first sample and the
+//     masks of the intervals that end inside the run, so the interval of every
+//     sample is a running count; each sample gathers its interval's four
+//     coefficients from L1 with one vector load per envelope.  All loads of a
+//     run are independent of one another and there is no branch, so they and
+//     the evaluations overlap; the sample's offset in its interval is 1 right
+//     after a knot and grows by 1, both exact;
 //   - new values and SD partials; strict extrema of the new values with lane
 //     neighbours by shuffle; the tile's last sample is decided with the next
 //     tile (its right neighbour), so only the two samples just outside the
@@ -930,10 +904,19 @@ __device__ T outside_g(const Ctx& C, const TaskSm& S, const TaskDesc& d, const S
 //     samples, knots and this step's run records are written.
 // Every step reads one set of buffers and writes another (ping-pong), so the
 // warps of a step never see each other's writes.
+//
+// The sweep is bound by instruction issue and by the latency of its dependent
+// chains, not by traffic, hence registers instead of staging, gathers instead
+// of branches and 4-byte run records (they were 16 bytes, a third of the
+// step's traffic).  k_emd with samples staged in shared memory, records of 32
+// or 48 bytes loaded in a divergent branch per sample and knots compacted in
+// shared memory, against this form (B200): 48 000 samples x 100 trials
+// float32 5.77 -> 3.95 ms, 48 000 x 64 float64 1.71 -> 1.19 ms, 2^22 x 64
+// float64 505 -> 348 ms, one 8192-sample float64 EMD 0.331 -> 0.262 ms.
 template <typename T, bool EXACT, int MODE, int NW>
-__device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X, unsigned char* smem) {
+__device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X) {
     using G = Geo<T>;
-    constexpr int RUN = G::RUN, WT = G::WT, RS = G::RS;
+    constexpr int RUN = G::RUN, WT = G::WT;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr bool SIFTING = (MODE == TM_SIFT || MODE == TM_LAST);
     constexpr bool USES_R = (MODE == TM_LAST || MODE == TM_TRANS);
@@ -960,29 +943,29 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X, unsigned
         if (MODE == TM_TRANS && !S.imf_from_resid) io.hsrc = io.hdst;  // the sift that stopped wrote it
         io.trans_imf = (MODE == TM_TRANS) && (S.imf_from_resid || wd == 1);
     }
-    const int4* ri_cur = sl.ri + (int64_t)S.kpar * C.slot_runs;
-    int4* ri_nxt = sl.ri + (int64_t)(S.kpar ^ 1) * C.slot_runs;
+    const bool va_h = aligned32(io.hsrc), va_r = aligned32(io.rcur), va_i = aligned32(io.imf_m);
+    const bool va_o = aligned32(MODE == TM_SIFT ? io.hdst : io.rnxt);
+    const uint32_t* ri_cur = sl.ri + (int64_t)S.kpar * C.slot_runs;
+    uint32_t* ri_nxt = sl.ri + (int64_t)(S.kpar ^ 1) * C.slot_runs;
     const int np = S.kpar ^ 1;
     const int seg = rank * NW + wid;
     const int64_t pmx = knot_index(C, np, 0, seg, 0);
-    const int64_t pmn = knot_index(C, np, 1, seg, 0);
-    const T* R0 = static_cast<const T*>(sl.M);
-    const T* R1 = R0 + (int64_t)C.kcap * RS;
-    const int kbase0 = S.pref[S.kpar][0][seg], kbase1 = S.pref[S.kpar][1][seg];
+    const int pmd = (int)(knot_index(C, np, 1, seg, 0) - pmx);  // the minima's list from the maxima's
+    const Rec<T> R0(sl.M, 0, C.kcap), R1(sl.M, 1, C.kcap);
     // the warp's range [r0, r1): an equal share of the segment in whole runs
     // (shares in whole tiles left the last tiles' warps up to a tile behind),
     // cut into tiles of WT samples from r0 (the last one partial)
     const int nrun = (s1 - s0 + RUN - 1) / RUN;
     const int r0 = min(s1, s0 + (int)((int64_t)wid * nrun / NW) * RUN);
     const int r1 = min(s1, s0 + (int)((int64_t)(wid + 1) * nrun / NW) * RUN);
-    const int ta = 0, tb = (r1 - r0 + WT - 1) / WT;
-
-    unsigned char* wb = smem + (size_t)wid * G::WARP_BYTES;
-    T* const tbuf = reinterpret_cast<T*>(wb);                      // [2 buf][2 stream][TB]
-    int4* const rib = reinterpret_cast<int4*>(wb + G::TB_BYTES);  // [2 buf][32]
-    // the tile's new knots, compacted in time order before one coalesced copy out
-    int* const kts = reinterpret_cast<int*>(wb + G::TB_BYTES + G::RI_BYTES);  // [kind][KCAP]
-    T* const kvs = reinterpret_cast<T*>(wb + G::TB_BYTES + G::RI_BYTES + 2 * G::KCAP * 4);
+    const int tb = (r1 - r0 + WT - 1) / WT;
+    // real knots before the current tile (of the lists this step reads)
+    int kb0 = S.pref[S.kpar][0][seg], kb1 = S.pref[S.kpar][1][seg];
+    const int mir0 = S.mir[0], mir1 = S.mir[1];
+    const int hi0 = max(0, S.p2[0] - 2), hi1 = max(0, S.p2[1] - 2);  // last intervals
+    // no interval of the range is clipped at the signal's ends
+    const bool inner = kb0 + mir0 >= 1 && kb1 + mir1 >= 1 && S.pref[S.kpar][0][seg + 1] + mir0 - 1 <= hi0 &&
+                       S.pref[S.kpar][1][seg + 1] + mir1 - 1 <= hi1;
     double num = 0.0, den = 0.0;
 #ifdef EEMD_TRACE
     unsigned long long scyc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -999,194 +982,171 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X, unsigned
     } while (0)
 #endif
 
-    // tile j's samples [t0, t1) and run records into buffer b
-    // tile j's samples and run records live in ring buffer (j - ta) mod NBUF;
-    // NBUF - 1 tiles are in flight while one is processed
-    auto bufi = [&](int j) { return (j - ta) % G::NBUF; };
-    auto prefetch = [&](int j) {
-        const int t0 = r0 + j * WT, t1 = min(r1, t0 + WT), bi = bufi(j);
-        if (needs_h) tile_copy<T>(tbuf + (bi * 2) * G::TB, io.hsrc + t0, t1 - t0, lane);
-        if (USES_R) tile_copy<T>(tbuf + (bi * 2 + 1) * G::TB, io.rcur + t0, t1 - t0, lane);
-        if (SIFTING && lane * RUN < t1 - t0) cp_async16(rib + bi * 32 + lane, ri_cur + t0 / RUN + lane);
-        cp_async_commit();
+    // the next tile's runs and run records, in flight while a tile is processed
+    T hn[RUN], rn[RUN];
+    uint32_t rin = 0;
+    auto fetch = [&](int j) {
+        const int t = r0 + j * WT + lane * RUN;
+        const int nv = max(0, min(RUN, r1 - t));
+        if (needs_h) load_run<T, RUN>(io.hsrc + t, hn, nv, va_h);
+        if (USES_R) load_run<T, RUN>(io.rcur + t, rn, nv, va_r);
+        if (SIFTING) rin = nv > 0 ? ri_cur[t / RUN] : 0u;
     };
 
-    int wcx = 0, wcy = 0;  // knots of each kind written to the warp's lists so far
-    T gm1 = (T)0, gm2 = (T)0;  // next-knot values at t0-1 and t0-2 of the current tile
-    int cpx = 0, cpn = 0, cmask = 0, crun = 0, cbit = 0;  // run record awaiting its last sample
-    if (ta < tb) {
-        for (int q = 0; q < G::NBUF - 1 && ta + q < tb; ++q) prefetch(ta + q);
+    int wcx = 0, wcy = 0;      // knots of each kind written to the warp's lists so far
+    T gm1, gm2;                // next-knot values at t0-1 and t0-2 of the current tile
+    uint32_t prec = 0;         // this lane's run record of the previous tile, not written yet
+    gm1 = gm2 = (T)__int_as_float(0x7fc00000);  // NaN: the signal's first sample is no extremum
+    if (tb > 0) {
+        fetch(0);
         if (r0 > 0) {
             // the sample before the range: its value is the left neighbour of the range's first sample
             int c0 = 0, c1 = 0;
             if (SIFTING && lane == 0) {
-                const unsigned pm = (unsigned)__ldcg(&ri_cur[r0 / RUN - 1].z);
-                c0 = kbase0 - (int)((pm >> (RUN - 1)) & 1u);
-                c1 = kbase1 - (int)((pm >> (16 + RUN - 1)) & 1u);
+                const uint32_t pm = __ldcg(&ri_cur[r0 / RUN - 1]);
+                c0 = kb0 - (int)((pm >> (16 + RUN - 1)) & 1u);
+                c1 = kb1 - (int)((pm >> (24 + RUN - 1)) & 1u);
             }
             if (lane == 0) gm1 = outside_g<T, EXACT, MODE>(C, S, d, io, R0, R1, r0 - 1, c0, c1);
             gm1 = __shfl_sync(FULL, gm1, 0);
         }
     }
 
-    for (int j = ta; j < tb; ++j) {
-        const int t0 = r0 + j * WT, t1 = min(r1, t0 + WT), tl = t1 - t0;
-        const int j0 = lane * RUN;
-        const int nv = max(0, min(RUN, tl - j0));  // valid samples of this lane's run
-        const int last_lane = (tl - 1) / RUN;
-        const int b = bufi(j);
-        // tile j's copies are complete when at most the later tiles' groups
-        // (up to NBUF - 2 of them) are still pending
-        const int later = min(G::NBUF - 2, tb - 1 - j);
-        if (later >= 2) cp_async_wait<2>();
-        else if (later == 1) cp_async_wait<1>();
-        else cp_async_wait<0>();
-        __syncwarp();
-        if (j + G::NBUF - 1 < tb) prefetch(j + G::NBUF - 1);
-        SUB(0);
-        const T* hb = tbuf + (b * 2) * G::TB;
-        const T* rb = tbuf + (b * 2 + 1) * G::TB;
-        // (samples past the run's end are read but never used)
+    for (int j = 0; j < tb; ++j) {
+        const int t0 = r0 + j * WT, tl = min(WT, r1 - t0);
+        const int tj = t0 + lane * RUN;                  // first sample of this lane's run
+        const int nv = max(0, min(RUN, tl - lane * RUN));  // samples of the run
+        const bool whole = tl == WT;
+        const int last_lane = whole ? 31 : (tl - 1) / RUN;
         T hv[RUN], rv[RUN], fv[RUN], gv[RUN];
 #pragma unroll
-        for (int i = 0; i < RUN; ++i) hv[i] = rv[i] = fv[i] = gv[i] = (T)0;
-        if (nv > 0) {
-            if (needs_h) load_run<T, RUN>(hb + j0, hv);
-            if (USES_R) load_run<T, RUN>(rb + j0, rv);
+        for (int i = 0; i < RUN; ++i) {
+            hv[i] = needs_h ? hn[i] : (T)0;
+            rv[i] = USES_R ? rn[i] : (T)0;
         }
+        const uint32_t ri = rin;
+        if (j + 1 < tb) fetch(j + 1);
+        SUB(0);
 
         // ---------------- new values ----------------
         if (SIFTING) {
-            unsigned kmx = 0u, kmn = 0u;
-            int kb0 = 0, kb1 = 0;
-            if (nv > 0) {
-                const int4 ri = rib[b * 32 + lane];
-                kmx = (unsigned)ri.z & 0xffffu;
-                kmn = (unsigned)ri.z >> 16;
-                kb0 = kbase0 + ri.x;
-                kb1 = kbase1 + ri.y;
-            }
-            // interior tile: every sample's interval is (knots before it) + mir - 1, no clipping
-            const int ta0 = t0 + j0, ta1 = t0 + j0 + nv - 1;
-            bool ok = S.P[0] >= 2 && S.P[1] >= 2;
-#pragma unroll
-            for (int env = 0; env < 2; ++env) {
-                const int kb = env ? kb1 : kb0;
-                const int kc = __popc(env ? kmn : kmx);
-                const int mir = S.mir[env];
-                ok = ok && (!mir || (S.tfirst[env] < ta0 && S.tlast[env] >= ta1));
-                ok = ok && (kb + mir >= 1) && (kb + kc + mir <= S.p2[env] - 1);
-            }
-            const bool fast = __all_sync(FULL, ok || nv == 0);
-            T tnum = (T)0, tden = (T)0;  // fast mode: this tile's SD partial sums
-            // sample i of the run from its envelope mean m: new h, SD terms, next-knot value
-            auto finish = [&](int i, T m) {
-                const T h = hv[i];
-                const T hn = h - m;
-                fv[i] = hn;
-                if (EXACT) {
-                    const double dd = (C.rules == EEMD_RULES_NUMBA) ? (double)m : (double)(h - hn);
-                    num = num + dd * dd;
-                    den = den + (double)h * (double)h;
-                } else {
-                    const T dd = (C.rules == EEMD_RULES_NUMBA) ? m : h - hn;
-                    tnum = fmat(dd, dd, tnum);
-                    tden = fmat(h, h, tden);
-                }
-                gv[i] = (MODE == TM_LAST) ? rv[i] - hn : hn;
-            };
-            if (fast) {
-                // current and next interval of each envelope; the next record is
-                // loaded as soon as the current one is entered
-                Iv<T> c0, n0, c1, n1;
-                c0.t0 = c0.t1 = 0;
-                c0.y0 = c0.c1 = c0.c2 = c0.c3 = c0.y1 = c0.m1 = (T)0;
-                n0 = c1 = n1 = c0;
-                int k0 = kb0 + S.mir[0] - 1, k1 = kb1 + S.mir[1] - 1;
-                if (nv > 0) {
-                    // the interior test above keeps every index of the run in [0, p2 - 2]
-                    EEMD_CHECK_IV(k0, S.p2[0] - 2 - (int)__popc(kmx));
-                    EEMD_CHECK_IV(k1, S.p2[1] - 2 - (int)__popc(kmn));
-                    load_iv<T, EXACT>(c0, R0, k0);
-                    load_iv<T, EXACT>(c1, R1, k1);
-                    if (kmx) load_iv<T, EXACT>(n0, R0, k0 + 1);
-                    if (kmn) load_iv<T, EXACT>(n1, R1, k1 + 1);
-                }
-#pragma unroll
-                for (int i = 0; i < RUN; ++i) {
-                    if (i > 0 && ((kmx >> (i - 1)) & 1u)) {
-                        c0 = n0;
-                        ++k0;
-                        if (kmx >> i) load_iv<T, EXACT>(n0, R0, k0 + 1);
-                    }
-                    if (i > 0 && ((kmn >> (i - 1)) & 1u)) {
-                        c1 = n1;
-                        ++k1;
-                        if (kmn >> i) load_iv<T, EXACT>(n1, R1, k1 + 1);
-                    }
-                    const int t = t0 + j0 + i;
-                    if (i < nv) finish(i, (T)0.5 * (iv_eval<T, EXACT>(c0, t) + iv_eval<T, EXACT>(c1, t)));
-                }
-            } else {
+            unsigned kmx = (ri >> 16) & 0xffu, kmn = ri >> 24;
+            const int c0 = kb0 + (int)(ri & 0xffu), c1 = kb1 + (int)((ri >> 8) & 0xffu);  // knots before the run
+            T m[RUN];  // mean envelope
+            if constexpr (EXACT) {
                 Iv<T> v0, v1;
                 v0.k = v1.k = -1;
-                int cl0 = kb0, cl1 = kb1;
+                int cl0 = c0, cl1 = c1;
 #pragma unroll
                 for (int i = 0; i < RUN; ++i) {
-                    const int t = t0 + j0 + i;
+                    m[i] = (T)0;
                     if (i < nv) {
-                        const T eu = env_at<T, EXACT>(C, S, v0, R0, 0, cl0, t);
-                        const T el = env_at<T, EXACT>(C, S, v1, R1, 1, cl1, t);
-                        finish(i, (T)0.5 * (eu + el));
+                        const T eu = env_at<T, EXACT>(S, v0, R0, 0, cl0, tj + i);
+                        const T el = env_at<T, EXACT>(S, v1, R1, 1, cl1, tj + i);
+                        m[i] = (T)0.5 * (eu + el);
                     }
                     cl0 += (kmx >> i) & 1u;
                     cl1 += (kmn >> i) & 1u;
                 }
+            } else {
+                int k0 = c0 + mir0 - 1, k1 = c1 + mir1 - 1;
+                unsigned m0 = kmx, m1 = kmn;  // samples after which the interval changes
+                if (!inner) {
+                    // clipped at the ends: the first knot (no mirror) starts no new interval, nor does the last
+                    if (k0 < 0) m0 &= m0 - 1u;
+                    if (k1 < 0) m1 &= m1 - 1u;
+                    k0 = min(max(k0, 0), hi0);
+                    k1 = min(max(k1, 0), hi1);
+                    if (m0 && k0 + (int)__popc(m0) > hi0) m0 ^= 0x80000000u >> __clz(m0);
+                    if (m1 && k1 + (int)__popc(m1) > hi1) m1 ^= 0x80000000u >> __clz(m1);
+                }
+                EEMD_CHECK_IV(k0, hi0 - (int)__popc(m0));
+                EEMD_CHECK_IV(k1, hi1 - (int)__popc(m1));
+                // offsets in the intervals; float32 counts them in integers (exact beyond 2^24 too)
+                using Off = typename std::conditional<sizeof(T) == 4, int, T>::type;
+                Off d0 = tj - R0.t[k0], d1 = tj - R1.t[k1];
+#pragma unroll
+                for (int i = 0; i < RUN; ++i) {
+                    if (i > 0) {
+                        const bool b0 = (m0 >> (i - 1)) & 1u, b1 = (m1 >> (i - 1)) & 1u;
+                        k0 += b0;
+                        k1 += b1;
+                        d0 = b0 ? 1 : d0 + 1;
+                        d1 = b1 ? 1 : d1 + 1;
+                    }
+                    const T e0 = (T)d0, e1 = (T)d1;
+                    T a0, a1, a2, a3, b0, b1, b2, b3;
+                    load_coef<T>(R0.c, k0, a0, a1, a2, a3);
+                    load_coef<T>(R1.c, k1, b0, b1, b2, b3);
+                    const T eu = fmat(e0, fmat(e0, fmat(e0, a3, a2), a1), a0);
+                    const T el = fmat(e1, fmat(e1, fmat(e1, b3, b2), b1), b0);
+                    m[i] = (T)0.5 * (eu + el);
+                }
+                if (!whole) {
+#pragma unroll
+                    for (int i = 0; i < RUN; ++i)
+                        if (i >= nv) m[i] = (T)0;  // (hv is 0 there too: no SD terms)
+                }
+            }
+            T tnum = (T)0, tden = (T)0;  // fast mode: this tile's SD partial sums
+#pragma unroll
+            for (int i = 0; i < RUN; ++i) {
+                const T h = hv[i];
+                const T hn_ = h - m[i];
+                fv[i] = hn_;
+                if (EXACT) {
+                    const double dd = (C.rules == EEMD_RULES_NUMBA) ? (double)m[i] : (double)(h - hn_);
+                    num = num + dd * dd;
+                    den = den + (double)h * (double)h;
+                } else {
+                    const T dd = (C.rules == EEMD_RULES_NUMBA) ? m[i] : h - hn_;
+                    tnum = fmat(dd, dd, tnum);
+                    tden = fmat(h, h, tden);
+                }
+                gv[i] = (MODE == TM_LAST) ? rv[i] - hn_ : hn_;
             }
             if (!EXACT) {
                 num += (double)tnum;
                 den += (double)tden;
             }
+            // the tile's knots: the last run's position and its own
+            const int kt = (int)((ri & 0xffu) + __popc(kmx)) | ((int)(((ri >> 8) & 0xffu) + __popc(kmn)) << 16);
+            const int kl = __shfl_sync(FULL, kt, last_lane);
+            kb0 += kl & 0xffff;
+            kb1 += kl >> 16;
         } else {
 #pragma unroll
-            for (int i = 0; i < RUN; ++i)
-                if (i < nv) plain_value<T, MODE>(C, S, d, t0 + j0 + i, hv[i], rv[i], fv[i], gv[i]);
+            for (int i = 0; i < RUN; ++i) {
+                fv[i] = gv[i] = (T)0;
+                if (i < nv) plain_value<T, MODE>(C, S, d, tj + i, hv[i], rv[i], fv[i], gv[i]);
+            }
         }
         SUB(1);
 
         // ---------------- strict extrema of the new values ----------------
         // lanes decide their own samples except the tile's last one (its right
-        // neighbour is the next tile's first sample); lane 0 decides the
-        // previous tile's last sample
+        // neighbour is the next tile's first sample): the previous tile's last
+        // sample is decided now
         const T up = __shfl_up_sync(FULL, gv[RUN - 1], 1);
         const T dn = __shfl_down_sync(FULL, gv[0], 1);
-        const T gprev = (lane == 0) ? gm1 : up;
-        // samples of the run that may be knots: inside the run, not the tile's
-        // last sample, and 1 <= t <= n-2
-        unsigned valid = (1u << nv) - 1u;
-        if (j0 + nv == tl && nv > 0) valid &= ~(1u << (nv - 1));
-        if (t0 + j0 == 0) valid &= ~1u;
-        {
-            const int lim = n - 2 - (t0 + j0);  // largest run index with t <= n-2
-            if (lim < RUN - 1) valid &= (lim < 0) ? 0u : ((2u << lim) - 1u);
-        }
-        unsigned nmx = 0u, nmn = 0u;
+        const T gfirst = __shfl_sync(FULL, gv[0], 0);
+        unsigned rise = 0u, fall = 0u;  // bit i: sample i above / below the one before it
 #pragma unroll
-        for (int i = 0; i < RUN; ++i) {
-            const T a = (i == 0) ? gprev : gv[(i + RUN - 1) % RUN];
-            const T c = (i + 1 < RUN) ? gv[(i + 1) % RUN] : dn;
-            const T v = gv[i];
-            nmx |= (unsigned)((v > a) & (v > c)) << i;
-            nmn |= (unsigned)((v < a) & (v < c)) << i;
+        for (int i = 0; i <= RUN; ++i) {
+            const T a = (i == 0) ? (lane == 0 ? gm1 : up) : gv[(i + RUN - 1) % RUN];
+            const T v = (i == RUN) ? dn : gv[i % RUN];
+            if (v > a) rise |= 1u << i;
+            if (v < a) fall |= 1u << i;
         }
-        nmx &= valid;
-        nmn &= valid;
-        unsigned dmx = 0u, dmn = 0u;  // the previous tile's last sample (lane 0)
-        if (lane == 0 && j > ta && t0 - 1 >= 1 && t0 - 1 <= n - 2) {
-            dmx = (gm1 > gm2 && gm1 > gv[0]) ? 1u : 0u;
-            dmn = (gm1 < gm2 && gm1 < gv[0]) ? 1u : 0u;
-        }
-        const int cnt = (int)(__popc(nmx) + dmx) | ((int)(__popc(nmn) + dmn) << 16);
+        // samples of the run that may be knots: inside the run, not the tile's last sample
+        unsigned valid = (1u << nv) - 1u;
+        if (lane == last_lane) valid >>= 1;
+        const unsigned nmx = rise & (fall >> 1) & valid, nmn = fall & (rise >> 1) & valid;
+        // the previous tile's last sample (the same in every lane)
+        const bool carry = j > 0;
+        const unsigned dmx = (carry && gm1 > gm2 && gm1 > gfirst) ? 1u : 0u;
+        const unsigned dmn = (carry && gm1 < gm2 && gm1 < gfirst) ? 1u : 0u;
+        const int cnt = (int)__popc(nmx) | ((int)__popc(nmn) << 16);
         int inc = cnt;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1198,117 +1158,82 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X, unsigned
         SUB(2);
 
         // ---------------- writes ----------------
-        // knots go to shared memory at their tile position, then to the warp's
-        // lists with one coalesced copy per kind
-        int px = exc & 0xffff, pn = exc >> 16;  // tile positions
-        if (lane == 0 && j > ta) {
-            // the previous tile's last sample and the run record that waited for it
-            if (dmx) {
-                kts[px] = t0 - 1;
-                kvs[px] = gm1;
-            }
-            if (dmn) {
-                kts[G::KCAP + pn] = t0 - 1;
-                kvs[G::KCAP + pn] = gm1;
-            }
-            ri_nxt[crun] = make_int4(cpx, cpn, cmask | (int)(dmx << cbit) | (int)(dmn << (16 + cbit)), 0);
-            px += (int)dmx;
-            pn += (int)dmn;
+        const int nx = (tot & 0xffff) + (int)dmx, nn = (tot >> 16) + (int)dmn;
+        if (carry) {
+            // the previous tile's run records: its last sample's bit is known now
+            if (lane == 31) prec |= (dmx << (16 + RUN - 1)) | (dmn << (24 + RUN - 1));
+            ri_nxt[t0 / RUN - 32 + lane] = prec;
         }
-        const int rpx = wcx + px, rpn = wcy + pn, rmask = (int)(nmx | (nmn << 16));
-        if (nv > 0 && lane != last_lane) ri_nxt[t0 / RUN + lane] = make_int4(rpx, rpn, rmask, 0);
-        {
-            // the run's new values go to the (already consumed) h tile buffer, so a
-            // knot's value is read by index; only the set bits are visited
-            T* const gsm = tbuf + (b * 2) * G::TB + j0;
-            store_run_smem<T, RUN>(gsm, gv);
-            for (unsigned m = nmx; m; m &= m - 1u) {
-                const int i = __ffs(m) - 1;
-                kts[px] = t0 + j0 + i;
-                kvs[px] = gsm[i];
-                ++px;
+        const int px = exc & 0xffff, pn = exc >> 16;  // positions within the tile
+        prec = run_record(px, pn, nmx, nmn);
+        if (wcx + nx > C.segcap || wcy + nn > C.segcap) {
+            if (lane == 0) task_error(C, S, EEMD_E_KNOT_OVERFLOW);
+        } else {
+            if (lane == 31) {
+                if (dmx) put_knot<T>(sl, pmx + wcx, t0 - 1, gm1);
+                if (dmn) put_knot<T>(sl, pmx + pmd + wcy, t0 - 1, gm1);
             }
-            for (unsigned m = nmn; m; m &= m - 1u) {
-                const int i = __ffs(m) - 1;
-                kts[G::KCAP + pn] = t0 + j0 + i;
-                kvs[G::KCAP + pn] = gsm[i];
-                ++pn;
-            }
-        }
-        __syncwarp();
-        {
-            const int nx = tot & 0xffff, nn = tot >> 16;
-            if (wcx + nx > C.segcap || wcy + nn > C.segcap || nx > G::KCAP || nn > G::KCAP) {
-                if (lane == 0) task_error(C, S, EEMD_E_KNOT_OVERFLOW);
-            } else {
-                T* const ky = static_cast<T*>(sl.ky);
-                for (int k = lane; k < nx; k += 32) {
-                    sl.kt[pmx + wcx + k] = kts[k];
-                    ky[pmx + wcx + k] = kvs[k];
-                }
-                for (int k = lane; k < nn; k += 32) {
-                    sl.kt[pmn + wcy + k] = kts[G::KCAP + k];
-                    ky[pmn + wcy + k] = kvs[G::KCAP + k];
+            if (tot) {
+                // straight to the lists: a run's knots of a kind are neighbours there, and so are the lanes'
+                int ox = wcx + (int)dmx + px, on = pmd + wcy + (int)dmn + pn;
+#pragma unroll
+                for (int i = 0; i < RUN; ++i) {
+                    const bool ax = (nmx >> i) & 1u, an = (nmn >> i) & 1u;
+                    const int o = ax ? ox : on;
+                    if (ax || an) put_knot<T>(sl, pmx + o, tj + i, gv[i]);
+                    ox += ax;
+                    on += an;
                 }
             }
         }
-        const int tj = t0 + j0;
         if (MODE == TM_SIFT) {
-            store_run<T, RUN>(io.hdst + tj, fv, nv);
+            store_run<T, RUN>(io.hdst + tj, fv, nv, va_o);
         } else if (MODE == TM_LAST) {
-            store_run<T, RUN>(io.imf_m + tj, fv, nv);
-            store_run<T, RUN>(io.rnxt + tj, gv, nv);
+            store_run<T, RUN>(io.imf_m + tj, fv, nv, va_i);
+            store_run<T, RUN>(io.rnxt + tj, gv, nv, va_o);
         } else if (MODE == TM_TRANS) {
-            store_run<T, RUN>(io.rnxt + tj, fv, nv);
+            store_run<T, RUN>(io.rnxt + tj, fv, nv, va_o);
             if (io.trans_imf) {
-                if (S.imf_from_resid) store_run<T, RUN>(io.imf_m + tj, rv, nv);
-                else store_run<T, RUN>(io.imf_m + tj, hv, nv);
+                if (S.imf_from_resid) store_run<T, RUN>(io.imf_m + tj, rv, nv, va_i);
+                else store_run<T, RUN>(io.imf_m + tj, hv, nv, va_i);
             }
         } else {
-            store_run<T, RUN>(io.rnxt + tj, fv, nv);
+            store_run<T, RUN>(io.rnxt + tj, fv, nv, va_o);
         }
-        // carry to the next tile: the last sample's neighbours and its run record
-        cpx = __shfl_sync(FULL, rpx, last_lane);
-        cpn = __shfl_sync(FULL, rpn, last_lane);
-        cmask = __shfl_sync(FULL, rmask, last_lane);
-        crun = t0 / RUN + last_lane;
-        cbit = tl - 1 - last_lane * RUN;
-        gm2 = (tl >= 2) ? tile_at<T, RUN>(gv, tl - 2) : gm1;
-        gm1 = tile_at<T, RUN>(gv, tl - 1);
-        wcx += tot & 0xffff;
-        wcy += tot >> 16;
+        // carry to the next tile: the last sample's value and its left neighbour's
+        if (whole) {
+            gm2 = __shfl_sync(FULL, gv[RUN - 2], 31);
+            gm1 = __shfl_sync(FULL, gv[RUN - 1], 31);
+        } else {
+            gm2 = (tl >= 2) ? tile_at<T, RUN>(gv, tl - 2) : gm1;
+            gm1 = tile_at<T, RUN>(gv, tl - 1);
+        }
+        wcx += nx;
+        wcy += nn;
         SUB(3);
     }
-    if (ta < tb) {
+    if (tb > 0) {
         // the range's last sample r1-1: its right neighbour lies outside the range
+        const int tlast = r0 + (tb - 1) * WT, last = r1 - 1 - tlast;  // last tile's start, r1-1 within it
         unsigned dmx = 0u, dmn = 0u;
-        if (lane == 0 && r1 < n && r1 - 1 >= 1) {
+        if (lane == 0 && r1 < n) {
             const T gr = outside_g<T, EXACT, MODE>(C, S, d, io, R0, R1, r1, S.pref[S.kpar][0][seg + 1],
                                                   S.pref[S.kpar][1][seg + 1]);
             dmx = (gm1 > gm2 && gm1 > gr) ? 1u : 0u;
             dmn = (gm1 < gm2 && gm1 < gr) ? 1u : 0u;
-        }
-        if (lane == 0) {
-            if (dmx) {
-                if (wcx < C.segcap) {
-                    sl.kt[pmx + wcx] = r1 - 1;
-                    static_cast<T*>(sl.ky)[pmx + wcx] = gm1;
-                } else {
-                    task_error(C, S, EEMD_E_KNOT_OVERFLOW);
-                }
+            if ((dmx && wcx >= C.segcap) || (dmn && wcy >= C.segcap)) {
+                task_error(C, S, EEMD_E_KNOT_OVERFLOW);
+            } else {
+                if (dmx) put_knot<T>(sl, pmx + wcx, r1 - 1, gm1);
+                if (dmn) put_knot<T>(sl, pmx + pmd + wcy, r1 - 1, gm1);
             }
-            if (dmn) {
-                if (wcy < C.segcap) {
-                    sl.kt[pmn + wcy] = r1 - 1;
-                    static_cast<T*>(sl.ky)[pmn + wcy] = gm1;
-                } else {
-                    task_error(C, S, EEMD_E_KNOT_OVERFLOW);
-                }
-            }
-            ri_nxt[crun] = make_int4(cpx, cpn, cmask | (int)(dmx << cbit) | (int)(dmn << (16 + cbit)), 0);
         }
-        wcx += (int)__shfl_sync(FULL, dmx, 0);
-        wcy += (int)__shfl_sync(FULL, dmn, 0);
+        dmx = __shfl_sync(FULL, dmx, 0);
+        dmn = __shfl_sync(FULL, dmn, 0);
+        if (lane == last / RUN) prec |= (dmx << (16 + last % RUN)) | (dmn << (24 + last % RUN));
+        if (lane <= last / RUN) ri_nxt[tlast / RUN + lane] = prec;
+        wcx += (int)dmx;
+        wcy += (int)dmn;
     }
     if (lane == 0) {
         X[q].cnt[0][wid] = wcx;
@@ -1528,7 +1453,7 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm(NW, (int)sizeof(T))) k_em
     const int slot = blockIdx.x / csize;
     const int tid = threadIdx.x;
     Slot sl;
-    sl.kt = C.kt + (int64_t)slot * C.slot_knots;
+    sl.kt = C.kt + (int64_t)slot * C.slot_knots * (sizeof(T) == 4 ? 2 : 1);
     sl.ky = static_cast<T*>(C.ky) + (int64_t)slot * C.slot_knots;
     sl.M = static_cast<T*>(C.M) + (int64_t)slot * C.slot_M;
     sl.w1 = static_cast<T*>(C.w1) + (int64_t)slot * C.slot_n;
@@ -1613,10 +1538,10 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm(NW, (int)sizeof(T))) k_em
                 EEMD_PHASE(2);
             }
             switch (S.mode) {
-                case TM_SIFT: sweep<T, EXACT, TM_SIFT, NW>(C, sl, S, X, smem_raw); break;
-                case TM_LAST: sweep<T, EXACT, TM_LAST, NW>(C, sl, S, X, smem_raw); break;
-                case TM_TRANS: sweep<T, EXACT, TM_TRANS, NW>(C, sl, S, X, smem_raw); break;
-                default: sweep<T, EXACT, TM_INIT, NW>(C, sl, S, X, smem_raw); break;
+                case TM_SIFT: sweep<T, EXACT, TM_SIFT, NW>(C, sl, S, X); break;
+                case TM_LAST: sweep<T, EXACT, TM_LAST, NW>(C, sl, S, X); break;
+                case TM_TRANS: sweep<T, EXACT, TM_TRANS, NW>(C, sl, S, X); break;
+                default: sweep<T, EXACT, TM_INIT, NW>(C, sl, S, X); break;
             }
             EEMD_PHASE(3);
             cl.sync();  // segment results published
@@ -2145,7 +2070,7 @@ int32_t eemd_run_traced(const eemd_params* p, const void* x, const int64_t* leng
     C.M = base + L.o_M;
     C.w1 = base + L.o_w1;
     C.r1 = base + L.o_r1;
-    C.ri = reinterpret_cast<int4*>(base + L.o_ri);
+    C.ri = reinterpret_cast<uint32_t*>(base + L.o_ri);
     C.scr = reinterpret_cast<double2*>(base + L.o_scr);
     C.x = x;
     C.noise = noise;

@@ -50,13 +50,6 @@ constexpr int MAXC = 16;
 #define EEMD_FAST_B 5
 #endif
 constexpr int FAST_B = EEMD_FAST_B;
-// warp tiles of samples in flight per sweep warp (a ring of buffers: the
-// copies of the next TILE_BUFS - 1 tiles run while one tile is processed)
-#ifndef EEMD_TILE_BUFS
-#define EEMD_TILE_BUFS 2
-#endif
-constexpr int TILE_BUFS = EEMD_TILE_BUFS;
-static_assert(TILE_BUFS >= 2 && TILE_BUFS <= 4, "two to four tile buffers");
 #ifndef EEMD_WSCAP
 #define EEMD_WSCAP 352
 #endif
@@ -115,13 +108,14 @@ struct Ctx {
     void* resid;                  // residual per task (dtype)
     void* imfs;                   // IMF slots per task (dtype)
     int32_t* kt;                  // per slot: [2 parity][2 env][C seg][segcap] knot sample index
-    void* ky;                     // per slot: same layout, knot value (dtype)
-    void* M;                      // per slot: [2 env][5][kcap] interval records (mirror space,
-                                  //   storage type): plane 0 = t_k; fast: monomial c0..c3 of
-                                  //   interval [k, k+1]; exact: y_k, M_k
+                                  //   (float32: pairs of index and value, kt and ky's space together)
+    void* ky;                     // per slot: same layout, knot value (float64)
+    void* M;                      // per slot: interval records (mirror space): [2 env][kcap] vectors
+                                  //   of four (fast: the monomial of interval [k, k+1]; exact: y_k,
+                                  //   M_k), then the knots' sample indices [2 env][kcap]
     void* w1;                     // per slot: scratch h buffer [slot_n] (storage type)
     void* r1;                     // per slot: second residual buffer [slot_n] (storage type)
-    int4* ri;                     // per slot: run records [2 parity][slot_runs]
+    uint32_t* ri;                 // per slot: run records [2 parity][slot_runs]
     double2* scr;                 // exact-mode solve scratch: [rows][grid threads]
     const void* x;
     const void* noise;

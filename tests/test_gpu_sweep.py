@@ -1,0 +1,83 @@
+"""The sweep at the edges of its tiling, against the oracle's emd_1d
+(emd_ref.py:108-156): a warp tile is 32 runs of 8 float32 or 4 float64
+samples, each warp of a task owns whole runs of its CTA's segment, and rows
+that do not start on 32 bytes are read and written by element."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+pytest.importorskip("torch")
+
+from eemd4cuda_b200 import emd_par as M  # noqa: E402
+
+# one sample to one side and the other of a run, a tile (128 and 256), a
+# warp's share of 4 and 5 warps, and lengths that leave rows misaligned
+LENGTHS = [127, 128, 129, 255, 256, 257, 511, 513, 1025, 1283, 2047, 2050, 4099]
+
+
+def rows_of(lengths, seed):
+    rng = np.random.default_rng(seed)
+    out = []
+    for n in lengths:
+        t = np.arange(n, dtype=float)
+        out.append(np.sin(2 * np.pi * t / 23.0) + 0.4 * np.sin(2 * np.pi * t / 6.1) + 0.3 * rng.standard_normal(n))
+    return out
+
+
+def end_rows():
+    """Few knots: every interval of most tiles is clipped at the signal's ends;
+    the last row has a single maximum (a constant upper envelope)."""
+    n = 3001
+    t = np.arange(n, dtype=float)
+    one = np.minimum(np.sin(2 * np.pi * t / 700.0), 0.5)
+    one += 0.7 * np.exp(-((t - 1575.0) / 30.0) ** 2)
+    return [np.sin(2 * np.pi * t / 1300.0), np.sin(2 * np.pi * (t + 200) / 420.0) + 1e-4 * t, one]
+
+
+def check(rows, tol, **kw):
+    from oracle import emd_oracle as O
+    from test_gpu_parity import engine_log, max_imf_err, oracle_log, raw_run
+
+    dtype = kw.get("dtype", np.float64)
+    rows = [r.astype(dtype).astype(np.float64) for r in rows]
+    args = dict(tau=0.0, max_sifts=kw["max_sifts"], max_imf=kw["max_imf"], end=kw["end"])
+    res = raw_run(None, x=np.concatenate(rows), lengths=[len(r) for r in rows], trial_count=1, exact=False,
+                  dtype=dtype, config=kw["config"], **args)
+    for k, row in enumerate(rows):
+        imfs, resid, st = O.emd_1d(row, record_knots=True, **args)
+        assert int(res["nmode"][k]) == st["n_modes"], len(row)
+        assert engine_log(res, k) == oracle_log(st), len(row)
+        scale = np.abs(row).max()
+        assert max_imf_err(res["imfs"][k][:st["n_modes"]], imfs, scale) <= tol, len(row)
+        assert np.max(np.abs(res["resid"][k] - resid)) <= tol * scale * max(1, st["n_modes"]), len(row)
+
+
+@pytest.mark.parametrize("end", ["natural", "mirror"])
+@pytest.mark.parametrize("cta_warps", [4, 5])
+@pytest.mark.parametrize("csize", [1, 2])
+def test_tile_edges_float64(end, cta_warps, csize):
+    """Six sifts of up to six IMFs: knot counts of every sift equal, values
+    within the seam-window solve's 1e-9 of max|x|."""
+    lengths = LENGTHS if csize == 1 else [n for n in LENGTHS if n >= 256]
+    cfg = M.EngineConfig(cluster_size=csize, cta_warps=cta_warps)
+    check(rows_of(lengths, 11), 1e-9, max_sifts=6, max_imf=6, end=end, config=cfg)
+
+
+@pytest.mark.parametrize("end", ["natural", "mirror"])
+@pytest.mark.parametrize("cta_warps", [4, 5])
+def test_tile_edges_float32(end, cta_warps):
+    """One sift, so that no float32 rounding can move a knot: the envelopes'
+    coefficients and Horner steps are rounded to 2^-24 of terms of the order
+    of ten max|x| at most, which stays within 1e-5 of max|x|."""
+    cfg = M.EngineConfig(cluster_size=1, cta_warps=cta_warps)
+    check(rows_of(LENGTHS, 12), 1e-5, max_sifts=1, max_imf=1, end=end, dtype=np.float32, config=cfg)
+
+
+@pytest.mark.parametrize("end", ["natural", "mirror"])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_clipped_intervals(end, dtype):
+    """Long stretches before the first and after the last knot, and an
+    envelope of a single knot (bounds as above)."""
+    cfg = M.EngineConfig(cluster_size=1, cta_warps=4)
+    check(end_rows(), 1e-9 if dtype == np.float64 else 1e-5, max_sifts=1, max_imf=1, end=end, dtype=dtype,
+          config=cfg)
