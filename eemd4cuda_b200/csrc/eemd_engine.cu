@@ -265,16 +265,6 @@ struct Geo {
 
 __host__ __device__ inline int stage_pad(int k) { return k + (k >> 4); }
 
-// Staging slot of knot k.  The lanes of a solve pass read knots one window
-// width apart: exact windows (16 knots) pad one slot every 16 so that the
-// lanes spread over the banks; fast windows of an odd width already hit 32
-// distinct banks unpadded (stride 3 is a permutation of the 32 banks, and of
-// the 16 bank pairs of a half-warp's doubles), and padding would collide them.
-template <bool EXACT>
-__host__ __device__ inline int stage_slot(int k) {
-    return (EXACT || FAST_B % 2 == 0) ? stage_pad(k) : k;
-}
-
 __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
 
 // rows of one fast-solve pass: 32 lanes of FAST_B rows
@@ -283,18 +273,24 @@ constexpr int FAST_ROWS = 32 * FAST_B;
 // its rows, the left halo and the two knots past the last row
 constexpr int FAST_SMAX = 64;
 constexpr int WSCAP_FAST = FAST_ROWS + FAST_SMAX + 3;
+static_assert(WSCAP_FAST <= 2 * FAST_ROWS, "the slopes of a pass fit the (c, d) area");
 
-// knots a solve pass stages per warp: exact windows carry both halos (up to
-// WSCAP knots); the fast solve's lanes need WSCAP_FAST
-__host__ __device__ constexpr int stage_cap(bool exact) { return exact ? WSCAP : WSCAP_FAST; }
-
-// per-warp solve area: slopes (double), knot times (int), knot values
-// (storage type), and in fast mode the forward (c, d) of a pass's rows.  What
-// it leaves of the SM's on-chip memory is L1, which the sweep's record
-// gathers live in.
+// Per-warp staging area of the solve.  What the CTAs' areas leave of the SM's
+// on-chip memory is L1, which the sweep's record gathers live in.
+//   exact: slopes (double), knot times (int) and values (double) of WSCAP
+//     knots, one slot of padding every 16 (the lanes of a pass read knots one
+//     window of 16 apart, which would share a bank);
+//   fast: the rows (diagonal, right-hand side) and the knots (float32: pairs
+//     of time and value; float64: times, then values) of WSCAP_FAST knots, and
+//     the forward (c, d) of a pass's rows, whose space first holds the slopes.
+//     Lanes read FAST_B elements apart: odd strides hit distinct banks.
 __host__ __device__ inline size_t wsolve_bytes(size_t bt, bool exact) {
-    const size_t sp = (size_t)stage_pad(stage_cap(exact));
-    return align16(sp * 8) + align16(sp * 4) + align16(sp * bt) + (exact ? 0 : (size_t)FAST_ROWS * 16);
+    if (exact) {
+        const size_t sp = (size_t)stage_pad(WSCAP);
+        return align16(sp * 8) + align16(sp * 4) + align16(sp * 8);
+    }
+    return (size_t)WSCAP_FAST * 16 + align16((size_t)WSCAP_FAST * 4) + align16((size_t)WSCAP_FAST * bt) + 16 +
+           (size_t)FAST_ROWS * 16;
 }
 
 // dynamic shared memory of k_emd: the solve's per-warp areas (the sweep works in registers)
@@ -367,29 +363,28 @@ __device__ __forceinline__ void real_knot(const Ctx& C, const Slot& sl, const Ta
     y = (double)v;
 }
 
-// Stage the mirror-space knots rlo .. rlo+kcount-1 (lane-strided); each lane
-// finds the segment of its first real knot by binary search and then walks
-// forward, since its later knots follow in the same or later segments.
-template <typename T, bool EXACT>
-__device__ __forceinline__ void stage_range(const Ctx& C, const Slot& sl, TaskSm& S, int env, int rlo,
-                                            int kcount, int* skt, T* sky, int lane) {
+// Exact mode: stage the mirror-space knots rlo .. rlo+kcount-1 (lane-strided);
+// each lane finds the segment of its first real knot by binary search and then
+// walks forward, since its later knots follow in the same or later segments.
+__device__ __forceinline__ void stage_exact(const Ctx& C, const Slot& sl, TaskSm& S, int env, int rlo, int kcount,
+                                            int* skt, double* sky, int lane) {
     const int* pr = S.pref[S.kpar][env];
     const int nseg = S.csize * C.nw;
     const int mir = S.mir[env], P = S.P[env];
     int r = -1;
     for (int k = lane; k < kcount; k += 32) {
         int i2 = rlo + k;
-        int* kt_s = &skt[stage_slot<EXACT>(k)];
-        T* ky_s = &sky[stage_slot<EXACT>(k)];
+        int* kt_s = &skt[stage_pad(k)];
+        double* ky_s = &sky[stage_pad(k)];
         if (mir) {
             if (i2 == 0) {
                 *kt_s = S.tfirst[env];
-                *ky_s = (T)S.yfirst[env];
+                *ky_s = S.yfirst[env];
                 continue;
             }
             if (i2 == P + 1) {
                 *kt_s = S.tlast[env];
-                *ky_s = (T)S.ylast[env];
+                *ky_s = S.ylast[env];
                 continue;
             }
             i2 -= 1;
@@ -403,12 +398,104 @@ __device__ __forceinline__ void stage_range(const Ctx& C, const Slot& sl, TaskSm
         }
 #endif
         const int64_t o = knot_index(C, S.kpar, env, r, i2 - pr[r]);
+        cp_async4(kt_s, sl.kt + o);
+        cp_async8(ky_s, static_cast<const double*>(sl.ky) + o);
+    }
+}
+
+// Staged knots of the fast solve
+template <typename T>
+struct Knots {
+    int* t;     // float32: pairs (time, value bits); float64: times
+    double* v;  // float64: values
+    __device__ __forceinline__ int time(int k) const { return sizeof(T) == 4 ? t[2 * k] : t[k]; }
+    __device__ __forceinline__ T val(int k) const {
+        if constexpr (sizeof(T) == 4) return __int_as_float(t[2 * k + 1]);
+        else return v[k];
+    }
+    __device__ __forceinline__ void get(int k, int& tk, T& y) const {
         if constexpr (sizeof(T) == 4) {
-            cp_async4(kt_s, sl.kt + 2 * o);
-            cp_async4(ky_s, sl.kt + 2 * o + 1);
+            const int2 p = reinterpret_cast<const int2*>(t)[k];
+            tk = p.x;
+            y = __int_as_float(p.y);
         } else {
-            cp_async4(kt_s, sl.kt + o);
-            cp_async8(ky_s, static_cast<const T*>(sl.ky) + o);
+            tk = t[k];
+            y = v[k];
+        }
+    }
+    __device__ __forceinline__ void set(int k, int tk, T y) const {
+        if constexpr (sizeof(T) == 4) {
+            reinterpret_cast<int2*>(t)[k] = make_int2(tk, __float_as_int(y));
+        } else {
+            t[k] = tk;
+            v[k] = y;
+        }
+    }
+    __device__ __forceinline__ void copy(int k, const Slot& sl, int64_t o) const {  // asynchronously
+        if constexpr (sizeof(T) == 4) {
+            cp_async8(t + 2 * k, sl.kt + 2 * o);
+        } else {
+            cp_async4(t + k, sl.kt + o);
+            cp_async8(v + k, static_cast<const double*>(sl.ky) + o);
+        }
+    }
+};
+
+// Fast mode: stage the mirror-space knots rlo .. rlo+kcount-1.  The real knots
+// among them lie in consecutive (CTA, warp) segments: up to STAGE_PIECES
+// segments are copied piece by piece (a pass of dense knots spans one or two),
+// more by a lane-strided walk as in stage_exact (the sparse knots of the late
+// IMFs, a few per segment).
+constexpr int STAGE_PIECES = 4;
+template <typename T>
+__device__ __forceinline__ void stage_fast(const Ctx& C, const Slot& sl, TaskSm& S, int env, int rlo, int kcount,
+                                           const Knots<T>& K, int lane) {
+    const int* pr = S.pref[S.kpar][env];
+    const int nseg = S.csize * C.nw;
+    const int mir = S.mir[env], P = S.P[env];
+    if (mir && lane == 0) {
+        if (rlo == 0) K.set(0, S.tfirst[env], (T)S.yfirst[env]);
+        if (rlo + kcount == P + 2) K.set(kcount - 1, S.tlast[env], (T)S.ylast[env]);
+    }
+    int a = max(rlo - mir, 0);                       // real knots [a, b)
+    const int b = min(rlo + kcount - mir, P);
+    const int shift = mir - rlo;                     // staging position of real knot i: i + shift
+    // segments of the first and last knot: the last one that starts at or before it
+    int ra = 0, rb = 0;
+#pragma unroll
+    for (int k = 0; k < (MAXSEG + 31) / 32; ++k) {
+        const int sg = 32 * k + lane;
+        const int v = sg < nseg ? pr[sg] : INT_MAX;
+        ra += __popc(__ballot_sync(0xffffffffu, v <= a));
+        rb += __popc(__ballot_sync(0xffffffffu, v <= b - 1));
+    }
+    ra -= 1;
+    rb -= 1;
+    if (rb - ra < STAGE_PIECES) {
+        for (int r = ra; r <= rb; ++r) {
+            const int e = min(b, pr[r + 1]);
+            const int64_t o = knot_index(C, S.kpar, env, r, 0) - pr[r];
+#ifdef EEMD_CHECKED
+            if (a < pr[r] || e - pr[r] > C.segcap || a + shift < 0 || e + shift > WSCAP_FAST) {
+                task_error(C, S, EEMD_E_KNOT_OVERFLOW);
+                return;
+            }
+#endif
+            for (int i = a + lane; i < e; i += 32) K.copy(i + shift, sl, o + i);
+            a = e;
+        }
+    } else {
+        int r = -1;
+        for (int i = a + lane; i < b; i += 32) {
+            if (r < 0) r = seg_of(pr, 0, nseg, i);
+            while (r + 1 < nseg && i >= pr[r + 1]) ++r;
+#ifdef EEMD_CHECKED
+            if (i - pr[r] >= C.segcap || i + shift < 0 || i + shift >= WSCAP_FAST) {
+                task_error(C, S, EEMD_E_KNOT_OVERFLOW);
+                continue;
+            }
+#endif
+            K.copy(i + shift, sl, knot_index(C, S.kpar, env, r, i - pr[r]));
         }
     }
 }
@@ -464,8 +551,8 @@ __device__ __forceinline__ Row row_of(int ta, int tb, int tc, double sa, double 
     return w;
 }
 
-#define SKT(k) skt[stage_slot<kExact>(k)]
-#define SSL(k) ssl[stage_slot<kExact>(k)]
+#define SKT(k) skt[stage_pad(k)]
+#define SSL(k) ssl[stage_pad(k)]
 
 // Interval records of one envelope in mirror space: for interval k (knots k,
 // k+1) the four coefficients c[4k..4k+3] (fast: y_k, c1, c2, c3 of the
@@ -497,7 +584,6 @@ struct Rec {
 template <typename T>
 __device__ void window_exact(const Ctx& C, const int* skt, const T* sky, const double* ssl, int base,
                              int n, int w, const Rec<T>& R, int p2) {
-    constexpr bool kExact = true;
     const int B = C.B, S = C.S;
     const int o0 = w * B;
     const int o1 = min(n, o0 + B) - 1;
@@ -522,7 +608,7 @@ __device__ void window_exact(const Ctx& C, const int* skt, const T* sky, const d
         sa = sb;
     }
     auto put = [&](int k, double Mk) {
-        R.put(k, SKT(k - base), sky[stage_slot<kExact>(k - base)], (T)Mk, (T)0, (T)0);
+        R.put(k, SKT(k - base), sky[stage_pad(k - base)], (T)Mk, (T)0, (T)0);
     };
     double xv = dp;
     if (w1 <= o1) put(w1 + 1, xv);
@@ -535,6 +621,9 @@ __device__ void window_exact(const Ctx& C, const int* skt, const T* sky, const d
     if (o1 == n - 1) put(p2 - 1, 0.0);
 }
 
+#undef SKT
+#undef SSL
+
 // fast: each lane owns FAST_B consecutive rows of a pass.  The forward
 // elimination (coupling dropped S rows before the lane's first row, where the
 // influence of the neglected rows has decayed like prod c_i) stores (c_i, d_i)
@@ -546,27 +635,41 @@ __device__ void window_exact(const Ctx& C, const int* skt, const T* sky, const d
 // (unless the pass reaches the envelope's last row) and are solved for good
 // by the next pass.  Per owned row: (S + FAST_B) / FAST_B eliminated rows and
 // as many back-substitution steps (one fused multiply-add each).
+//
+// A row is formed once per pass, by the lane that owns its knot, and read by
+// the (S + FAST_B) / FAST_B lanes that eliminate it: {d_i, r_i} in one 16-byte
+// load, with d_i = 2 (H_i + H_{i+1}) and r_i = 6 (slope_{i+1} - slope_i).  The
+// off-diagonals follow from d_i alone, H_{i+1} = d_i / 2 - H_i, exactly (they
+// are differences of sample indices).  The first and last row need no special
+// case: the terms their outer couplings multiply are zero.  The elimination is
+// a chain of dependent float64 operations at 13 to 16 warps per SM; forming a
+// row in every lane that eliminates it (three conversions and four operations
+// more per row, and two loads) made k_emd 48 000 x 100 float32 3.96 ms, this
+// form 3.53; 48 000 x 64 float64 1.19 and 1.10; 2^22 x 64 float64 349 and 330.
 template <typename T>
-__device__ __forceinline__ void window_fast_fwd(const int* skt, const double* ssl, int base, int n, int w, int S,
-                                                double2* cd, int cdbase) {
-    constexpr bool kExact = false;
+__device__ __forceinline__ void window_fast_fwd(const Knots<T>& K, const double2* rows, int base, int n, int w,
+                                                int S, double2* cd, int cdbase) {
     const int o0 = w * FAST_B;
     const int o1 = min(n, o0 + FAST_B) - 1;
     const int r0 = max(0, o0 - S);
     double cp = 0.0, dp = 0.0;
-    int ta = SKT(r0 - base), tb = SKT(r0 + 1 - base);
-    double sa = SSL(r0 - base);
-    for (int i = r0; i <= o1; ++i) {
-        const int tc = SKT(i + 2 - base);
-        const double sb = SSL(i + 1 - base);
-        const Row rw = row_of(ta, tb, tc, sa, sb, i, n);
-        const double inv = fast_rcp(fma(-rw.l, cp, rw.dg));
-        cp = rw.u * inv;
-        dp = fma(-rw.l, dp, rw.r) * inv;
-        if (i >= o0) cd[i - cdbase] = make_double2(cp, dp);
-        ta = tb;
-        tb = tc;
-        sa = sb;
+    double l = (double)(K.time(r0 + 1 - base) - K.time(r0 - base));  // H_i
+    auto step = [&](int i) {
+        const double2 rw = rows[i - base];
+        const double u = fma(0.5, rw.x, -l);
+        const double inv = fast_rcp(fma(-l, cp, rw.x));
+        dp = fma(-l, dp, rw.y) * inv;
+        cp = u * inv;
+        l = u;
+    };
+#pragma unroll 4
+    for (int i = r0; i < o0; ++i) step(i);
+#pragma unroll
+    for (int k = 0; k < FAST_B; ++k) {
+        if (o0 + k <= o1) {
+            step(o0 + k);
+            cd[o0 + k - cdbase] = make_double2(cp, dp);
+        }
     }
 }
 
@@ -574,34 +677,46 @@ __device__ __forceinline__ void window_fast_fwd(const int* skt, const double* ss
 // its interval records: interval i+1 for every owned row i (knots i+1, i+2),
 // and interval 0 (M_0 = 0 at the natural end) for the first window.
 template <typename T>
-__device__ __forceinline__ void window_fast_back(const int* skt, const T* sky, const double* ssl, int base, int n,
-                                                 int w, int S, const double2* cd, int cdbase, const Rec<T>& R) {
-    constexpr bool kExact = false;
+__device__ __forceinline__ void window_fast_back(const Knots<T>& K, int base, int n, int w, int S, const double2* cd,
+                                                 int cdbase, const Rec<T>& R) {
     const int o0 = w * FAST_B;
     const int o1 = min(n, o0 + FAST_B) - 1;
     const int rh = min(n - 1, o1 + S);
+    double xn = 0.0;  // x_{i+1}: zero past the natural end (M = 0) or at the truncation
+#pragma unroll 4
+    for (int i = rh; i > o1; --i) {
+        const double2 c = cd[i - cdbase];
+        xn = fma(-c.x, xn, c.y);
+    }
     // monomial record of interval k (knots k, k+1; M_k = Ma, M_{k+1} = Mb):
     // y_k + s(c1 + s(c2 + s c3)), s = t - t_k, c1 = slope - h(2Ma + Mb)/6,
     // c2 = Ma/2, c3 = (Mb - Ma)/(6h)
+    int t1;
+    T y1;
+    K.get(o1 + 2 - base, t1, y1);
     auto put = [&](int k, double Ma, double Mb) {
-        const int t0 = SKT(k - base), t1 = SKT(k + 1 - base);
-        const double h = (double)(t1 - t0);
-        R.put(k, t0, sky[stage_slot<kExact>(k - base)],
-              (T)fma(-h * (1.0 / 6.0), fma(2.0, Ma, Mb), SSL(k - base)), (T)(0.5 * Ma),
-              (T)((Mb - Ma) * fast_rcp(h) * (1.0 / 6.0)));
+        int t0;
+        T y0;
+        K.get(k - base, t0, y0);
+        const double h = (double)(t1 - t0), rh_ = fast_rcp(h);
+        const double slope = ((double)y1 - (double)y0) * rh_;
+        R.put(k, t0, y0, (T)fma(-h * (1.0 / 6.0), fma(2.0, Ma, Mb), slope), (T)(0.5 * Ma),
+              (T)((Mb - Ma) * rh_ * (1.0 / 6.0)));
+        t1 = t0;
+        y1 = y0;
     };
-    double xn = 0.0;  // x_{i+1}: zero past the natural end (M = 0) or at the truncation
-    for (int i = rh; i >= o0; --i) {
-        const double2 c = cd[i - cdbase];
-        const double xi = fma(-c.x, xn, c.y);
-        if (i <= o1) put(i + 1, xi, xn);
-        xn = xi;
+#pragma unroll
+    for (int k = FAST_B - 1; k >= 0; --k) {
+        const int i = o0 + k;
+        if (i <= o1) {
+            const double2 c = cd[i - cdbase];
+            const double xi = fma(-c.x, xn, c.y);
+            put(i + 1, xi, xn);
+            xn = xi;
+        }
     }
     if (o0 == 0) put(0, 0.0, xn);
 }
-
-#undef SKT
-#undef SSL
 
 template <typename T, bool EXACT, int NW>
 __device__ void solve_task(const Ctx& C, const Slot& sl, TaskSm& S, unsigned char* smem) {
@@ -646,13 +761,17 @@ __device__ void solve_task(const Ctx& C, const Slot& sl, TaskSm& S, unsigned cha
     const int ca = (int)((int64_t)S.rank * nwt / S.csize), cb = (int)((int64_t)(S.rank + 1) * nwt / S.csize);
     const int wa = ca + (int)((int64_t)wid * (cb - ca) / NW);
     const int wb = ca + (int)((int64_t)(wid + 1) * (cb - ca) / NW);
-    constexpr int CAP = stage_cap(EXACT);
     unsigned char* ws = smem + (size_t)wid * wsolve_bytes(sizeof(T), EXACT);
+    // exact: slopes, knot times, knot values
     double* ssl = reinterpret_cast<double*>(ws);
-    int* skt = reinterpret_cast<int*>(ws + align16(stage_pad(CAP) * 8));
-    T* sky = reinterpret_cast<T*>(ws + align16(stage_pad(CAP) * 8) + align16(stage_pad(CAP) * 4));
-    double2* cd = reinterpret_cast<double2*>(ws + align16(stage_pad(CAP) * 8) + align16(stage_pad(CAP) * 4) +
-                                             align16(stage_pad(CAP) * sizeof(T)));
+    int* skt = reinterpret_cast<int*>(ws + align16(stage_pad(WSCAP) * 8));
+    double* sky = reinterpret_cast<double*>(ws + align16(stage_pad(WSCAP) * 8) + align16(stage_pad(WSCAP) * 4));
+    // fast: rows, (c, d) or slopes, knots
+    double2* rows = reinterpret_cast<double2*>(ws);
+    double2* cd = rows + WSCAP_FAST;
+    Knots<T> K;
+    K.t = reinterpret_cast<int*>(cd + FAST_ROWS);
+    K.v = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(K.t) + align16((size_t)WSCAP_FAST * 4));
     // exact: windows of B rows with halos on both sides, one per lane;
     // fast: lanes of FAST_B rows, the last H lanes of a pass as right halo
     const int H = (C.S + FAST_B - 1) / FAST_B;
@@ -681,27 +800,45 @@ __device__ void solve_task(const Ctx& C, const Slot& sl, TaskSm& S, unsigned cha
             rhi = min(n - 1, (w0 + nl) * FAST_B - 1);
         }
         const int kcount = rhi + 3 - rlo;  // knots rlo .. rhi+2
-        stage_range<T, EXACT>(C, sl, S, env, rlo, kcount, skt, sky, lane);
-        cp_async_commit();
-        cp_async_wait<0>();
-        __syncwarp();
-        SUB(0);
-        for (int k = lane; k + 1 < kcount; k += 32) {
-            const int ta = skt[stage_slot<EXACT>(k)], tb = skt[stage_slot<EXACT>(k + 1)];
-            const double ya = (double)sky[stage_slot<EXACT>(k)], yb = (double)sky[stage_slot<EXACT>(k + 1)];
-            // emd_ref.py:47: (y_{q+1}-y_q)/H_q (the same IEEE division in exact mode)
-            ssl[stage_slot<EXACT>(k)] = EXACT ? (yb - ya) / (double)(tb - ta) : (yb - ya) * fast_rcp((double)(tb - ta));
-        }
-        __syncwarp();
-        SUB(1);
         const Rec<T> R(sl.M, env, C.kcap);
         const int w = w0 + lane;
-        if (EXACT) {
+        if constexpr (EXACT) {
+            stage_exact(C, sl, S, env, rlo, kcount, skt, sky, lane);
+            cp_async_commit();
+            cp_async_wait<0>();
+            __syncwarp();
+            SUB(0);
+            // emd_ref.py:47: (y_{q+1}-y_q)/H_q, the same IEEE division
+            for (int k = lane; k + 1 < kcount; k += 32)
+                ssl[stage_pad(k)] = (sky[stage_pad(k + 1)] - sky[stage_pad(k)]) /
+                                    (double)(skt[stage_pad(k + 1)] - skt[stage_pad(k)]);
+            __syncwarp();
+            SUB(1);
             if (lane < nl) window_exact<T>(C, skt, sky, ssl, rlo, n, w, R, p2);
         } else {
-            if (lane < nl) window_fast_fwd<T>(skt, ssl, rlo, n, w, C.S, cd, w0 * FAST_B);
+            stage_fast<T>(C, sl, S, env, rlo, kcount, K, lane);
+            cp_async_commit();
+            cp_async_wait<0>();
             __syncwarp();
-            if (lane < ncommit) window_fast_back<T>(skt, sky, ssl, rlo, n, w, C.S, cd, w0 * FAST_B, R);
+            SUB(0);
+            double* slope = reinterpret_cast<double*>(cd);
+            for (int k = lane; k + 1 < kcount; k += 32) {
+                int ta, tb;
+                T ya, yb;
+                K.get(k, ta, ya);
+                K.get(k + 1, tb, yb);
+                slope[k] = ((double)yb - (double)ya) * fast_rcp((double)(tb - ta));
+            }
+            __syncwarp();
+            for (int k = lane; k + 2 < kcount; k += 32) {
+                const double d = 2.0 * (double)(K.time(k + 2) - K.time(k));
+                rows[k] = make_double2(d, 6.0 * (slope[k + 1] - slope[k]));
+            }
+            __syncwarp();
+            SUB(1);
+            if (lane < nl) window_fast_fwd<T>(K, rows, rlo, n, w, C.S, cd, w0 * FAST_B);
+            __syncwarp();
+            if (lane < ncommit) window_fast_back<T>(K, rlo, n, w, C.S, cd, w0 * FAST_B, R);
         }
         __syncwarp();
         SUB(2);

@@ -75,9 +75,11 @@ def test_tile_edges_float32(end, cta_warps):
 
 @pytest.mark.parametrize("end", ["natural", "mirror"])
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
-def test_clipped_intervals(end, dtype):
+@pytest.mark.parametrize("csize", [1, 8])
+def test_clipped_intervals(end, dtype, csize):
     """Long stretches before the first and after the last knot, and an
-    envelope of a single knot (bounds as above)."""
-    cfg = M.EngineConfig(cluster_size=1, cta_warps=4)
+    envelope of a single knot (bounds as above); with eight CTAs the few knots
+    of a solve pass lie in more segments than are staged piece by piece."""
+    cfg = M.EngineConfig(cluster_size=csize, cta_warps=4)
     check(end_rows(), 1e-9 if dtype == np.float64 else 1e-5, max_sifts=1, max_imf=1, end=end, dtype=dtype,
           config=cfg)
