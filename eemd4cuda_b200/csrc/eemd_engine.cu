@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(1024) k_sigma(const SignalDesc* sdesc, const v
 // ---------------------------------------------------------------------------
 constexpr int MAXSEG = MAXC * MAXNW;  // knot segments per task: one per warp of up to MAXC CTAs
 
-struct Xchg {              // one CTA's published segment results (DSMEM-visible)
-    double num, den;       // SD partial sums of the segment
+struct Xchg {              // one CTA's published step results (DSMEM-visible)
+    double2 sd[MAXNW];     // SD partial sums (num, den) of each warp's range, where the stop test reads them
     int cnt[2][MAXNW];     // new knots (maxima, minima) found by each warp
     int err;               // this CTA raised an error during the step: the task stops
 };
@@ -220,21 +220,18 @@ struct TaskSm {
     int nsift_total, nmode, mode_sifts_cur, flags, step, mode;
     int P[2];                  // current knot totals
     int pref[2][2][MAXSEG + 1];  // [list parity][env]: knots before each (CTA, warp) segment
-    int mir[2], p2[2], tfirst[2], tlast[2];
-    double yfirst[2], ylast[2];  // values of the virtual mirror knots
-    double cval[2];            // constant envelope when P == 1
+    int mir[2], p2[2];         // mirror ends in use; knots in mirror space
     int rcur;                  // current residual: 0 = the task's residual array, 1 = slot scratch
-    int err;                   // this CTA raised an error during the current step
-    int setup_fail;            // step_setup found a capacity exceeded (identical in every CTA)
+    Xchg x[2];                 // step results, by step parity
 };
 
 // An error of the running task: recorded in the header (first error wins) and
-// in the CTA's step flag, which decide() ORs over the cluster so that every
+// in the CTA's step results, which decide() ORs over the cluster so that every
 // CTA stops the task at the same step (no further step reads what the failed
 // step left behind).
 __device__ __forceinline__ void task_error(const Ctx& C, TaskSm& S, int code) {
     raise_error(C.hdr, code, S.task);
-    S.err = 1;
+    S.x[S.step & 1].err = 1;
 }
 
 #ifdef EEMD_CHECKED
@@ -363,6 +360,28 @@ __device__ __forceinline__ void real_knot(const Ctx& C, const Slot& sl, const Ta
     y = (double)v;
 }
 
+// Mirror space (emd_ref.py:92-96): with mir = 1 (three knots or more) the list
+// is [2t0-t1, t0..t_{P-1}, 2t_{P-1}-t_{P-2}] with values [y1, y.., y_{P-2}].
+// The two virtual knots of a staged range are formed from their neighbours
+// once those have arrived (get, set: a staged knot).
+template <typename Get, typename Set>
+__device__ __forceinline__ void mirror_ends(const TaskSm& S, int env, int rlo, int kcount, int lane, Get get, Set set) {
+    if (!S.mir[env] || lane != 0) return;
+    if (rlo == 0) {
+        const auto a = get(1), b = get(2);
+        set(0, 2 * a.t - b.t, b.y);
+    }
+    if (rlo + kcount == S.P[env] + 2) {
+        const auto a = get(kcount - 2), b = get(kcount - 3);
+        set(kcount - 1, 2 * a.t - b.t, b.y);
+    }
+}
+template <typename T>
+struct KnotVal {
+    int t;
+    T y;
+};
+
 // Exact mode: stage the mirror-space knots rlo .. rlo+kcount-1 (lane-strided);
 // each lane finds the segment of its first real knot by binary search and then
 // walks forward, since its later knots follow in the same or later segments.
@@ -377,16 +396,7 @@ __device__ __forceinline__ void stage_exact(const Ctx& C, const Slot& sl, TaskSm
         int* kt_s = &skt[stage_pad(k)];
         double* ky_s = &sky[stage_pad(k)];
         if (mir) {
-            if (i2 == 0) {
-                *kt_s = S.tfirst[env];
-                *ky_s = S.yfirst[env];
-                continue;
-            }
-            if (i2 == P + 1) {
-                *kt_s = S.tlast[env];
-                *ky_s = S.ylast[env];
-                continue;
-            }
+            if (i2 == 0 || i2 == P + 1) continue;  // the virtual knots follow from their staged neighbours
             i2 -= 1;
         }
         if (r < 0) r = seg_of(pr, 0, nseg, i2);
@@ -453,10 +463,6 @@ __device__ __forceinline__ void stage_fast(const Ctx& C, const Slot& sl, TaskSm&
     const int* pr = S.pref[S.kpar][env];
     const int nseg = S.csize * C.nw;
     const int mir = S.mir[env], P = S.P[env];
-    if (mir && lane == 0) {
-        if (rlo == 0) K.set(0, S.tfirst[env], (T)S.yfirst[env]);
-        if (rlo + kcount == P + 2) K.set(kcount - 1, S.tlast[env], (T)S.ylast[env]);
-    }
     int a = max(rlo - mir, 0);                       // real knots [a, b)
     const int b = min(rlo + kcount - mir, P);
     const int shift = mir - rlo;                     // staging position of real knot i: i + shift
@@ -498,36 +504,6 @@ __device__ __forceinline__ void stage_fast(const Ctx& C, const Slot& sl, TaskSm&
             K.copy(i + shift, sl, knot_index(C, S.kpar, env, r, i - pr[r]));
         }
     }
-}
-
-// Knot i2 in "mirror space" (emd_ref.py:92-96): with mir=1 the list is
-// [2t0-t1, t0..t_{P-1}, 2t_{P-1}-t_{P-2}] with values [y1, y.., y_{P-2}].
-template <typename T>
-__device__ __forceinline__ void knot2(const Ctx& C, const Slot& sl, const TaskSm& S, int env, int i2,
-                                      int& t, double& y) {
-    const int P = S.P[env];
-    if (S.mir[env]) {
-        if (i2 == 0) {
-            int t0, t1;
-            double y0, y1;
-            real_knot<T>(C, sl, S, env, 0, t0, y0);
-            real_knot<T>(C, sl, S, env, 1, t1, y1);
-            t = 2 * t0 - t1;
-            y = y1;
-            return;
-        }
-        if (i2 == P + 1) {
-            int ta, tb;
-            double ya, yb;
-            real_knot<T>(C, sl, S, env, P - 1, ta, ya);
-            real_knot<T>(C, sl, S, env, P - 2, tb, yb);
-            t = 2 * ta - tb;
-            y = yb;
-            return;
-        }
-        i2 -= 1;
-    }
-    real_knot<T>(C, sl, S, env, i2, t, y);
 }
 
 // ---------------------------------------------------------------------------
@@ -742,10 +718,10 @@ __device__ void solve_task(const Ctx& C, const Slot& sl, TaskSm& S, unsigned cha
         const Rec<T> R(sl.M, env, C.kcap);
         int tk, t1;
         double yk, y1;
-        knot2<T>(C, sl, S, env, tid, tk, yk);
+        real_knot<T>(C, sl, S, env, tid, tk, yk);  // (no mirror knots below three)
         T c1 = (T)0;
         if (!EXACT && tid + 1 < p2) {
-            knot2<T>(C, sl, S, env, tid + 1, t1, y1);
+            real_knot<T>(C, sl, S, env, tid + 1, t1, y1);
             c1 = (T)((y1 - yk) / (double)(t1 - tk));
         }
         R.put(tid, tk, (T)yk, c1, (T)0, (T)0);
@@ -807,6 +783,13 @@ __device__ void solve_task(const Ctx& C, const Slot& sl, TaskSm& S, unsigned cha
             cp_async_commit();
             cp_async_wait<0>();
             __syncwarp();
+            mirror_ends(S, env, rlo, kcount, lane,
+                        [&](int k) { return KnotVal<double>{skt[stage_pad(k)], sky[stage_pad(k)]}; },
+                        [&](int k, int t, double y) {
+                            skt[stage_pad(k)] = t;
+                            sky[stage_pad(k)] = y;
+                        });
+            __syncwarp();
             SUB(0);
             // emd_ref.py:47: (y_{q+1}-y_q)/H_q, the same IEEE division
             for (int k = lane; k + 1 < kcount; k += 32)
@@ -820,6 +803,16 @@ __device__ void solve_task(const Ctx& C, const Slot& sl, TaskSm& S, unsigned cha
             cp_async_commit();
             cp_async_wait<0>();
             __syncwarp();
+            if (S.mir[env]) {
+                mirror_ends(S, env, rlo, kcount, lane,
+                            [&](int k) {
+                                KnotVal<T> v;
+                                K.get(k, v.t, v.y);
+                                return v;
+                            },
+                            [&](int k, int t, T y) { K.set(k, t, y); });
+                __syncwarp();
+            }
             SUB(0);
             double* slope = reinterpret_cast<double*>(cd);
             for (int k = lane; k + 1 < kcount; k += 32) {
@@ -844,7 +837,6 @@ __device__ void solve_task(const Ctx& C, const Slot& sl, TaskSm& S, unsigned cha
         SUB(2);
         g += ncommit;
     }
-    __syncthreads();
 #ifdef EEMD_TRACE
     if (lane == 0) {
         for (int k = 0; k < 3; ++k) atomicAdd(&C.hdr->sweep_cycles[4 + k], scyc[k]);
@@ -973,6 +965,12 @@ __device__ __forceinline__ uint32_t run_record(int px, int pn, unsigned mx, unsi
     return (uint32_t)px | ((uint32_t)pn << 8) | (mx << 16) | (mn << 24);
 }
 
+// whether the stop test reads the step's SD: from the second sift on, where a
+// sum of squares over another can fall below tau at all
+__device__ __forceinline__ bool reads_sd(const Ctx& C, const TaskSm& S) {
+    return S.mode == TM_SIFT && S.sift >= 1 && C.tau > 0.0;
+}
+
 // Pointers and flags of one sweep step.
 template <typename T>
 struct StepIo {
@@ -1051,14 +1049,13 @@ __device__ T outside_g(const Ctx& C, const TaskSm& S, const TaskDesc& d, const S
 // float32 5.77 -> 3.95 ms, 48 000 x 64 float64 1.71 -> 1.19 ms, 2^22 x 64
 // float64 505 -> 348 ms, one 8192-sample float64 EMD 0.331 -> 0.262 ms.
 template <typename T, bool EXACT, int MODE, int NW>
-__device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X) {
+__device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S) {
     using G = Geo<T>;
     constexpr int RUN = G::RUN, WT = G::WT;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr bool SIFTING = (MODE == TM_SIFT || MODE == TM_LAST);
     constexpr bool USES_R = (MODE == TM_LAST || MODE == TM_TRANS);
-    __shared__ double2 s_red[NW];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int n = S.n, s0 = S.s0, s1 = S.s1, rank = S.rank;
     const bool needs_h = SIFTING || (MODE == TM_TRANS && !S.imf_from_resid);
     const int q = S.step & 1;
@@ -1104,6 +1101,7 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X) {
     const bool inner = kb0 + mir0 >= 1 && kb1 + mir1 >= 1 && S.pref[S.kpar][0][seg + 1] + mir0 - 1 <= hi0 &&
                        S.pref[S.kpar][1][seg + 1] + mir1 - 1 <= hi1;
     double num = 0.0, den = 0.0;
+    const bool need_sd = reads_sd(C, S);
 #ifdef EEMD_TRACE
     unsigned long long scyc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     long long smark = clock64();
@@ -1119,7 +1117,13 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X) {
     } while (0)
 #endif
 
-    // the next tile's runs and run records, in flight while a tile is processed
+    // the next tile's runs and run records, in flight while a tile is
+    // processed.  At 128 registers they are asked for once the values are done
+    // and take the registers those leave (at the tile's start they spilled:
+    // k_emd many 32-trial signals 51.8 ms against 47.4, 48 000 x 100 float32
+    // 3.57 against 3.40); at 168 the earlier load covers more of the DRAM
+    // latency of long signals (2^22 x 64 float64 327 ms against 335)
+    constexpr bool FETCH_EARLY = !SIFTING || (sizeof(T) == 8 && NW == 4);
     T hn[RUN], rn[RUN];
     uint32_t rin = 0;
     auto fetch = [&](int j) {
@@ -1162,7 +1166,7 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X) {
             rv[i] = USES_R ? rn[i] : (T)0;
         }
         const uint32_t ri = rin;
-        if (j + 1 < tb) fetch(j + 1);
+        if (FETCH_EARLY && j + 1 < tb) fetch(j + 1);
         SUB(0);
 
         // ---------------- new values ----------------
@@ -1229,20 +1233,20 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X) {
 #pragma unroll
             for (int i = 0; i < RUN; ++i) {
                 const T h = hv[i];
-                const T hn_ = h - m[i];
-                fv[i] = hn_;
-                if (EXACT) {
-                    const double dd = (C.rules == EEMD_RULES_NUMBA) ? (double)m[i] : (double)(h - hn_);
-                    num = num + dd * dd;
-                    den = den + (double)h * (double)h;
-                } else {
-                    const T dd = (C.rules == EEMD_RULES_NUMBA) ? m[i] : h - hn_;
-                    tnum = fmat(dd, dd, tnum);
-                    tden = fmat(h, h, tden);
+                fv[i] = h - m[i];
+                gv[i] = (MODE == TM_LAST) ? rv[i] - fv[i] : fv[i];
+                if (MODE == TM_SIFT) {
+                    const T dd = (C.rules == EEMD_RULES_NUMBA) ? m[i] : h - fv[i];
+                    if (EXACT) {
+                        num = num + (double)dd * (double)dd;
+                        den = den + (double)h * (double)h;
+                    } else {
+                        tnum = fmat(dd, dd, tnum);
+                        tden = fmat(h, h, tden);
+                    }
                 }
-                gv[i] = (MODE == TM_LAST) ? rv[i] - hn_ : hn_;
             }
-            if (!EXACT) {
+            if (MODE == TM_SIFT && !EXACT) {
                 num += (double)tnum;
                 den += (double)tden;
             }
@@ -1251,6 +1255,7 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X) {
             const int kl = __shfl_sync(FULL, kt, last_lane);
             kb0 += kl & 0xffff;
             kb1 += kl >> 16;
+            if (!FETCH_EARLY && j + 1 < tb) fetch(j + 1);
         } else {
 #pragma unroll
             for (int i = 0; i < RUN; ++i) {
@@ -1372,9 +1377,17 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X) {
         wcx += (int)dmx;
         wcy += (int)dmn;
     }
+    if (MODE == TM_SIFT && need_sd) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            num += __shfl_down_sync(FULL, num, o);
+            den += __shfl_down_sync(FULL, den, o);
+        }
+    }
     if (lane == 0) {
-        X[q].cnt[0][wid] = wcx;
-        X[q].cnt[1][wid] = wcy;
+        S.x[q].cnt[0][wid] = wcx;
+        S.x[q].cnt[1][wid] = wcy;
+        if (MODE == TM_SIFT && need_sd) S.x[q].sd[wid] = make_double2(num, den);
     }
 #ifdef EEMD_TRACE
     if (lane == 0) {
@@ -1382,13 +1395,6 @@ __device__ void sweep(const Ctx& C, const Slot& sl, TaskSm& S, Xchg* X) {
     }
 #endif
 #undef SUB
-    // ---------------- publish the segment's SD partials ----------------
-    const double2 rs = block_sum2<32 * NW>(make_double2(num, den), s_red);
-    if (tid == 0) {
-        X[q].num = rs.x;
-        X[q].den = rs.y;
-        X[q].err = S.err;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1435,15 +1441,36 @@ __device__ __forceinline__ void imf_level(const Ctx& C, TaskSm& S, int cmax, int
     adopt(S, cmax, cmin);
 }
 
+// the next step's mode and envelopes (mirror ends from three knots on)
+__device__ __forceinline__ void set_step(const Ctx& C, TaskSm& S) {
+    if (S.phase == PH_TRANS) S.mode = TM_TRANS;
+    if (S.phase != PH_SIFT) return;
+    S.mode = (S.sift + 1 >= C.max_sifts) ? TM_LAST : TM_SIFT;
+    for (int env = 0; env < 2; ++env) {
+        S.mir[env] = (C.end_mode == EEMD_END_MIRROR && S.P[env] >= 3) ? 1 : 0;
+        S.p2[env] = S.P[env] + 2 * S.mir[env];
+        if (S.p2[env] > C.kcap) {
+            // computed from the same counts in every CTA of the cluster: all leave the task together
+            raise_error(C.hdr, EEMD_E_KNOT_OVERFLOW, S.task);
+            S.phase = PH_DONE;
+            S.flags |= 2;
+        }
+    }
+}
+
 // Warp 0 gathers the knot counts of every (CTA, warp) segment through
 // distributed shared memory and writes their prefixes for the new lists;
-// thread 0 then takes the step decision, identical in every CTA.
+// thread 0 then takes the step decision, identical in every CTA.  Every remote
+// read is one lane's: a step's critical path holds one round trip (the SD sums
+// and error flags read one CTA after another cost a round trip each).
 template <int NW>
-__device__ void decide(const Ctx& C, TaskSm& S, Xchg* X, cg::cluster_group& cl) {
+__device__ void decide(const Ctx& C, TaskSm& S, cg::cluster_group& cl) {
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         const int q = S.step & 1;
         const int nseg = S.csize * NW;
+        const bool need_sd = reads_sd(C, S);
+        const Xchg* X = &S.x[q];
         // segments SPL*lane .. SPL*lane + SPL-1 per lane (SPL = 3 covers the
         // 16 x 5 = 80 segments of the largest cluster of 5-warp CTAs)
         constexpr int SPL = (MAXSEG + 31) / 32;
@@ -1454,18 +1481,32 @@ __device__ void decide(const Ctx& C, TaskSm& S, Xchg* X, cg::cluster_group& cl) 
             const int sg = SPL * lane + k;
             c[0][k] = c[1][k] = 0;
             if (sg < nseg) {
-                const Xchg* xr = cl.map_shared_rank(&X[q], sg / NW);
+                const Xchg* xr = cl.map_shared_rank(X, sg / NW);
                 c[0][k] = xr->cnt[0][sg % NW];
                 c[1][k] = xr->cnt[1][sg % NW];
             }
         }
+        // one CTA's error flag and SD sums per lane, the warps' sums as a shuffle tree adds them
+        int err = 0;
+        double2 v = make_double2(0.0, 0.0);
+        if (lane < S.csize) {
+            const Xchg* xr = cl.map_shared_rank(X, lane);
+            err = xr->err;
+            if (need_sd) {
+                const double2 a = xr->sd[0], b = xr->sd[1], c2 = xr->sd[2], d = xr->sd[3];
+                const double2 e = NW == 5 ? xr->sd[NW - 1] : make_double2(0.0, 0.0);
+                v.x = ((a.x + e.x) + c2.x) + (b.x + d.x);
+                v.y = ((a.y + e.y) + c2.y) + (b.y + d.y);
+            }
+        }
+        err = __any_sync(0xffffffffu, err);
         int tot[2];
 #pragma unroll
         for (int env = 0; env < 2; ++env) {
-            int v = 0;
+            int sum = 0;
 #pragma unroll
-            for (int k = 0; k < SPL; ++k) v += c[env][k];
-            int inc = v;
+            for (int k = 0; k < SPL; ++k) sum += c[env][k];
+            int inc = sum;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int x = __shfl_up_sync(0xffffffffu, inc, o);
@@ -1473,7 +1514,7 @@ __device__ void decide(const Ctx& C, TaskSm& S, Xchg* X, cg::cluster_group& cl) 
             }
             tot[env] = __shfl_sync(0xffffffffu, inc, 31);
             int* pr = S.pref[S.kpar ^ 1][env];
-            int e = inc - v;
+            int e = inc - sum;
 #pragma unroll
             for (int k = 0; k < SPL; ++k) {
                 if (SPL * lane + k < nseg) pr[SPL * lane + k] = e;
@@ -1481,15 +1522,14 @@ __device__ void decide(const Ctx& C, TaskSm& S, Xchg* X, cg::cluster_group& cl) 
             }
             if (lane == 0) pr[nseg] = tot[env];
         }
-        if (lane == 0) {
-            double num = 0.0, den = 0.0;
-            int err = 0;
-            for (int r = 0; r < S.csize; ++r) {
-                const Xchg* xr = cl.map_shared_rank(&X[q], r);
-                num += xr->num;
-                den += xr->den;
-                err |= xr->err;
+        double num = 0.0, den = 0.0;
+        if (need_sd) {
+            for (int r = 0; r < S.csize; ++r) {  // in CTA order
+                num += __shfl_sync(0xffffffffu, v.x, r);
+                den += __shfl_sync(0xffffffffu, v.y, r);
             }
+        }
+        if (lane == 0) {
             const int cmax = tot[0], cmin = tot[1];
             const int mode = S.mode;
             if (err) {
@@ -1501,7 +1541,7 @@ __device__ void decide(const Ctx& C, TaskSm& S, Xchg* X, cg::cluster_group& cl) 
                 S.mode_sifts_cur += 1;
                 S.nsift_total += 1;
                 const double sdv = den > 0.0 ? num / den : 0.0;
-                bool stop = (S.sift >= 1) && (sdv < C.tau);
+                bool stop = need_sd && (sdv < C.tau);
                 if (!stop) stop = (C.rules == EEMD_RULES_NUMBA) ? (cmax < 2 || cmin < 2) : (cmax < 1 || cmin < 1);
                 if (stop) {
                     S.phase = PH_TRANS;
@@ -1529,47 +1569,14 @@ __device__ void decide(const Ctx& C, TaskSm& S, Xchg* X, cg::cluster_group& cl) 
                 imf_level(C, S, cmax, cmin);
             }
             S.step += 1;
+            // (its last readers, of the step before, have passed a cluster barrier since)
+            S.x[S.step & 1].err = 0;
+            set_step(C, S);
             // every IMF ends after at most max_sifts sifts plus one closing step
             if (S.phase != PH_DONE && S.step > 2 + C.max_imf * (C.max_sifts + 1)) {
                 raise_error(C.hdr, EEMD_E_TIMEOUT, S.task);
                 S.phase = PH_DONE;
             }
-        }
-    }
-    __syncthreads();
-}
-
-// per-step constants of the envelopes (mirror knots, constant envelope)
-template <typename T>
-__device__ void step_setup(const Ctx& C, const Slot& sl, TaskSm& S) {
-    if (threadIdx.x < 2) {
-        const int env = threadIdx.x;
-        const int P = S.P[env];
-        const int mir = (C.end_mode == EEMD_END_MIRROR && P >= 3) ? 1 : 0;
-        S.mir[env] = mir;
-        S.p2[env] = P + 2 * mir;
-        S.cval[env] = 0.0;
-        S.tfirst[env] = S.tlast[env] = 0;
-        if (P >= 1) {
-            int t0;
-            double y0;
-            real_knot<T>(C, sl, S, env, 0, t0, y0);
-            if (P == 1) S.cval[env] = y0;
-            if (mir) {
-                int t1, ta, tb;
-                double y1, ya, yb;
-                real_knot<T>(C, sl, S, env, 1, t1, y1);
-                real_knot<T>(C, sl, S, env, P - 1, ta, ya);
-                real_knot<T>(C, sl, S, env, P - 2, tb, yb);
-                S.tfirst[env] = 2 * t0 - t1;
-                S.tlast[env] = 2 * ta - tb;
-                S.yfirst[env] = y1;
-                S.ylast[env] = yb;
-            }
-        }
-        if (S.p2[env] > C.kcap) {
-            raise_error(C.hdr, EEMD_E_KNOT_OVERFLOW, S.task);
-            S.setup_fail = 1;  // computed from the same counts in every CTA of the cluster
         }
     }
     __syncthreads();
@@ -1582,7 +1589,6 @@ template <typename T, bool EXACT, int NW>
 __global__ void __launch_bounds__(32 * NW, ctas_per_sm(NW, (int)sizeof(T))) k_emd(const __grid_constant__ Ctx C) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ TaskSm S;
-    __shared__ Xchg X[2];
     __shared__ int s_claim;
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
@@ -1618,6 +1624,8 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm(NW, (int)sizeof(T))) k_em
         cl.sync();
         EEMD_PHASE(6);
         if (q >= C.n_tasks) break;
+        for (int r = tid; r <= MAXSEG; r += 32 * NW)
+            S.pref[0][0][r] = S.pref[0][1][r] = S.pref[1][0][r] = S.pref[1][1][r] = 0;
         if (tid == 0) {
             const int task = C.order[q];
             const TaskDesc d = C.td[task];
@@ -1631,9 +1639,9 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm(NW, (int)sizeof(T))) k_em
             S.imf = S.sift = S.kpar = S.src_resid = S.imf_from_resid = 0;
             S.nsift_total = S.nmode = S.mode_sifts_cur = S.flags = S.step = 0;
             S.P[0] = S.P[1] = 0;
-            for (int r = 0; r <= MAXSEG; ++r)
-                S.pref[0][0][r] = S.pref[0][1][r] = S.pref[1][0][r] = S.pref[1][1][r] = 0;
-            S.mir[0] = S.mir[1] = 0;
+            S.mir[0] = S.mir[1] = S.p2[0] = S.p2[1] = 0;
+            S.mode = TM_INIT;
+            S.x[0].err = S.x[1].err = 0;
             S.rcur = 1;  // the first step writes the residual array
             if (C.watchdog < 0 && rank == 0) {
                 // watchdog test mode: a bounded wait on a flag nothing sets
@@ -1649,25 +1657,7 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm(NW, (int)sizeof(T))) k_em
         }
         __syncthreads();
         while (S.phase != PH_DONE) {
-            if (tid == 0) {
-                if (S.phase == PH_INIT) S.mode = TM_INIT;
-                else if (S.phase == PH_TRANS) S.mode = TM_TRANS;
-                else S.mode = (S.sift + 1 >= C.max_sifts) ? TM_LAST : TM_SIFT;
-                S.err = 0;
-                S.setup_fail = 0;
-            }
-            __syncthreads();
             if (S.mode == TM_SIFT || S.mode == TM_LAST) {
-                step_setup<T>(C, sl, S);
-                if (S.setup_fail) {
-                    // every CTA of the cluster sees the same counts and leaves together
-                    if (tid == 0) {
-                        S.phase = PH_DONE;
-                        S.flags |= 2;
-                    }
-                    __syncthreads();
-                    break;
-                }
                 EEMD_PHASE(0);
                 solve_task<T, EXACT, NW>(C, sl, S, smem_raw);
                 EEMD_PHASE(1);
@@ -1675,15 +1665,15 @@ __global__ void __launch_bounds__(32 * NW, ctas_per_sm(NW, (int)sizeof(T))) k_em
                 EEMD_PHASE(2);
             }
             switch (S.mode) {
-                case TM_SIFT: sweep<T, EXACT, TM_SIFT, NW>(C, sl, S, X); break;
-                case TM_LAST: sweep<T, EXACT, TM_LAST, NW>(C, sl, S, X); break;
-                case TM_TRANS: sweep<T, EXACT, TM_TRANS, NW>(C, sl, S, X); break;
-                default: sweep<T, EXACT, TM_INIT, NW>(C, sl, S, X); break;
+                case TM_SIFT: sweep<T, EXACT, TM_SIFT, NW>(C, sl, S); break;
+                case TM_LAST: sweep<T, EXACT, TM_LAST, NW>(C, sl, S); break;
+                case TM_TRANS: sweep<T, EXACT, TM_TRANS, NW>(C, sl, S); break;
+                default: sweep<T, EXACT, TM_INIT, NW>(C, sl, S); break;
             }
             EEMD_PHASE(3);
             cl.sync();  // segment results published
             EEMD_PHASE(4);
-            decide<NW>(C, S, X, cl);
+            decide<NW>(C, S, cl);
             EEMD_PHASE(5);
         }
         if (S.rcur) {
