@@ -1173,6 +1173,213 @@ __global__ void __launch_bounds__(NT) k_wgrad_tc(const __nv_bfloat16* __restrict
     }
 }
 
+// Warp-specialised weight gradient for 16 or 64 input channels (CX) and 16 or
+// 64 output channels (NY), the form the training step runs.  The GEMM's K is
+// time, so both operands lie in memory with their rows along K: a tap of x is
+// the bulk-tensor box {CX channels, 128 samples} (shifted by the tap's dilation,
+// zero-filled outside [0, T)) and dy the box {NY, 128}, each in the swizzle its
+// row length has (128-byte or 32-byte), and the MMA reads them as MN-major
+// operands -- no transposition by threads, which took 90 of k_wgrad_tc's 100 us.
+// Consecutive taps are one tile apart, the MN-block stride of the descriptor:
+// rows of the A operand are (tap, channel), taps 0 and 1 of 64 channels in the
+// first accumulator and tap 2 in the second (its other 64 rows read what lies
+// behind and are not used), all three taps of 16 channels in one.
+//   copy warp : tile k into stage k mod NS once it is released (empty[s])
+//   MMA warp  : waits full[s], issues the tile's 8 or 16 MMAs, commits to
+//               empty[s]; after the last tile to accf
+//   4 warps   : add the tile's dy rows up for the bias gradient (in float32, on
+//               CUDA cores) and release the stage; after the last tile read the
+//               accumulators and add them to dw
+// Bound by the L2 traffic of four boxes per tile.  32 x 4096 samples, 64 to 64
+// channels: 100 us with k_wgrad_tc, 19.5 us here.  Every wait is bounded.
+constexpr int WG_SUM = 4;                       // summing warps
+constexpr int WG_THREADS = 32 * (WG_SUM + 2);
+
+template <int CX, int NY>
+struct WgGeo {
+    static constexpr int KT = 128;                        // samples per tile
+    static constexpr int XROW = CX * 2, YROW = NY * 2;    // bytes of a sample
+    static constexpr int XB = KT * XROW, YB = KT * YROW;  // bytes of a tap's tile, of dy's tile
+    static constexpr int STAGE = 3 * XB + YB;
+    static constexpr int NACC = CX == 64 ? 2 : 1;
+    static constexpr int NS = CX == 64 && NY == 64 ? 3 : 4;
+    // the A operand reaches 128 rows from its first tap: past the last stage's end
+    static constexpr int REACH = (CX == 64 ? 2 * XB : 0) + (128 / CX) * XB;
+    static constexpr int PAD = REACH > STAGE ? REACH - STAGE : 0;
+    static constexpr int SMEM = NS * STAGE + PAD + 1024;  // + alignment slack
+    static constexpr int TCOLS = NACC * NY < 32 ? 32 : NACC * NY;
+    static constexpr uint64_t XLAY = CX == 64 ? 2 : 6, YLAY = NY == 64 ? 2 : 6;  // 128-byte / 32-byte swizzle
+    static_assert(STAGE % 1024 == 0 && XB % 1024 == 0 && SMEM <= 227 * 1024, "tiles on swizzle boundaries");
+};
+
+// descriptor of an MN-major swizzled operand: blocks of one row length along MN
+// lbo bytes apart, groups of 8 samples along K sbo bytes apart
+__device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t lbo, uint32_t sbo, uint64_t layout) {
+    return smem_desc(addr, lbo, sbo) | (layout << 61);
+}
+
+template <int CX, int NY>
+__global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constant__ CUtensorMap tx,
+                                                             const __grid_constant__ CUtensorMap ty, float* dw,
+                                                             float* db, int B, int T, int nv, int cv, int dil, int* err,
+                                                             long long spin_limit) {
+    using G = WgGeo<CX, NY>;
+    constexpr int NS = G::NS;
+    constexpr uint32_t IDESC = instr_desc(128, NY) | (1u << 15) | (1u << 16);  // both operands MN-major
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t full[NS], empty[NS], accf;
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_flag;
+    __shared__ float sdb[NY];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    const unsigned char* const sm = smem_raw + (base - raw);
+    if (tid < NY) sdb[tid] = 0.f;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(G::TCOLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    if (tid == 0) {
+        for (int i = 0; i < NS; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&full[i])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&empty[i])), "n"(1 + WG_SUM));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&accf)));
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const int tiles_per_b = (T + G::KT - 1) / G::KT;
+    const int n_tiles = B * tiles_per_b;
+    const int nk = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+
+    if (warp == WG_SUM) {
+        // ---------------- copy warp ----------------
+        if (lane == 0) {
+            int k = 0;
+            for (; k < nk && !abort_flag; ++k) {
+                const int s = k % NS;
+                if (k >= NS && !wait_parity(&empty[s], (uint32_t)((k / NS) - 1) & 1u, spin_limit)) {
+                    raise(err, EEMD_SG_E_TIMEOUT);
+                    abort_flag = 1;
+                    break;
+                }
+                const int tile = blockIdx.x + k * gridDim.x;
+                const int b = tile / tiles_per_b, t0 = (tile % tiles_per_b) * G::KT;
+                const uint32_t dst = base + s * G::STAGE;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(&full[s])),
+                             "n"(G::STAGE)
+                             : "memory");
+#pragma unroll
+                for (int tap = 0; tap < 4; ++tap)  // (the fourth box is dy)
+                    asm volatile(
+                        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], "
+                        "[%1, {%2, %3, %4}], [%5];\n" ::"r"(dst + tap * G::XB),
+                        "l"(tap < 3 ? reinterpret_cast<uint64_t>(&tx) : reinterpret_cast<uint64_t>(&ty)), "r"(0),
+                        "r"(tap < 3 ? t0 + (tap - 1) * dil : t0), "r"(b), "r"(smem_u32(&full[s]))
+                        : "memory");
+            }
+            // copies still in flight (only when a role gave up) land before the CTA leaves
+            for (int j = k - 1; j >= 0 && j >= k - NS; --j) wait_parity(&full[j % NS], (uint32_t)(j / NS) & 1u, spin_limit);
+        }
+    } else if (warp == WG_SUM + 1) {
+        // ---------------- MMA warp ----------------
+        if (lane == 0) {
+            int k = 0;
+            for (; k < nk && !abort_flag; ++k) {
+                const int s = k % NS;
+                if (!wait_parity(&full[s], (uint32_t)(k / NS) & 1u, spin_limit)) {
+                    raise(err, EEMD_SG_E_TIMEOUT);
+                    abort_flag = 1;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint32_t st = base + s * G::STAGE;
+#pragma unroll
+                for (int j = 0; j < G::NACC; ++j) {
+#pragma unroll
+                    for (int q = 0; q < G::KT / 16; ++q) {
+                        const uint64_t da = mn_desc(st + j * 2 * G::XB + q * 16 * G::XROW, G::XB, 8 * G::XROW, G::XLAY);
+                        const uint64_t dd = mn_desc(st + 3 * G::XB + q * 16 * G::YROW, G::YB, 8 * G::YROW, G::YLAY);
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + j * NY),
+                            "l"(da), "l"(dd), "r"(IDESC), "r"(k > 0 || q > 0 ? 1u : 0u));
+                    }
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                                 smem_u32(&empty[s]))
+                             : "memory");
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                             smem_u32(&accf))
+                         : "memory");
+            // the issued MMAs are complete before the tensor memory is freed
+            wait_parity(&accf, 0u, spin_limit);
+        }
+    } else {
+        // ---------------- summing warps ----------------
+        constexpr int CH = NY / 8;                  // 16-byte chunks of a sample
+        constexpr int STEP = 32 * WG_SUM / CH;      // samples between a thread's rows
+        const int c = tid % CH, r0 = tid / CH;
+        float sum[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum[i] = 0.f;
+        bool ok = true;
+        for (int k = 0; k < nk && ok; ++k) {
+            const int s = k % NS;
+            ok = __all_sync(0xffffffffu, wait_parity(&full[s], (uint32_t)(k / NS) & 1u, spin_limit)) && !abort_flag;
+            if (!ok) break;
+            const unsigned char* y = sm + s * G::STAGE + 3 * G::XB;
+#pragma unroll
+            for (int r = r0; r < G::KT; r += STEP) {
+                const int pc = NY == 64 ? c ^ (r & 7) : c ^ ((r >> 2) & 1);
+                const uint4 v = *reinterpret_cast<const uint4*>(y + r * G::YROW + (pc << 4));
+                const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) sum[i] += __bfloat162float(h[i]);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[s]);
+        }
+        ok = __all_sync(0xffffffffu, ok && wait_parity(&accf, 0u, spin_limit)) && !abort_flag;
+        if (!ok) {
+            if (lane == 0) raise(err, EEMD_SG_E_TIMEOUT);
+            abort_flag = 1;
+        } else if (nk > 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) atomicAdd(&sdb[8 * c + i], sum[i]);
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < G::NACC; ++j) {
+                const int m0 = 128 * j + 32 * warp;  // this warp's rows (tap, channel) of the accumulator
+                if (m0 >= 3 * CX) continue;
+                float v[NY];
+                tmem_ld<NY>(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(j * NY), v);
+                const int m = m0 + lane, tap = m / CX, ch = m % CX;
+                if (m < 3 * CX && ch < cv) {
+#pragma unroll
+                    for (int n = 0; n < NY; ++n)
+                        if (n < nv) atomicAdd(&dw[((size_t)n * 3 + tap) * cv + ch], v[n]);
+                }
+            }
+        }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (!abort_flag && nk > 0 && tid < NY && tid < nv) atomicAdd(&db[tid], sdb[tid]);
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(G::TCOLS));
+    }
+}
+
 // prediction = base + out (residual form; base may be null) over the first
 // `cv` of `C` channels; loss partial sums over the interior [margin, T - margin)
 // and the gradient d loss / d out as bf16.  The loss per element is d^2 for
@@ -1186,36 +1393,51 @@ __global__ void k_loss(const __nv_bfloat16* __restrict__ out, const __nv_bfloat1
                        const __nv_bfloat16* __restrict__ target, __nv_bfloat16* dout, float* loss, int B, int T,
                        int C, int cv, int margin, float inv_count, int project, float delta,
                        const float* __restrict__ wch) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in_range = i < (long long)B * T * C;
-    float l = 0.f, g = 0.f;
-    int c = 0;
-    if (in_range) {
-        c = (int)(i % C);
-        const int t = (int)((i / C) % T);
-        if (c < cv && t >= margin && t < T - margin) {
-            const float d = (base ? __bfloat162float(base[i]) : 0.f) + __bfloat162float(out[i]) -
-                            __bfloat162float(target[i]);
-            const float wc = wch ? wch[c] : 1.f;
-            if (delta > 0.f && fabsf(d) > delta) {
-                l = wc * (2.f * delta * fabsf(d) - delta * delta);
-                g = 2.f * wc * copysignf(delta, d) * inv_count;
-            } else {
-                l = wc * d * d;
-                g = 2.f * wc * d * inv_count;
+    __shared__ float part[8];
+    const long long n = (long long)B * T * C;
+    float lsum = 0.f;
+    // (every lane of a warp takes part in each turn: the projection's shuffles)
+    for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < n; i0 += (long long)gridDim.x * blockDim.x) {
+        const long long i = i0 + threadIdx.x;
+        const bool in_range = i < n;
+        float l = 0.f, g = 0.f;
+        int c = 0;
+        if (in_range) {
+            const long long row = n <= 0xffffffffLL ? (long long)((uint32_t)i / (uint32_t)C) : i / C;
+            c = (int)(i - row * C);
+            const int t = n <= 0xffffffffLL ? (int)((uint32_t)row % (uint32_t)T) : (int)(row % T);
+            if (c < cv && t >= margin && t < T - margin) {
+                const float d = (base ? __bfloat162float(base[i]) : 0.f) + __bfloat162float(out[i]) -
+                                __bfloat162float(target[i]);
+                const float wc = wch ? wch[c] : 1.f;
+                if (delta > 0.f && fabsf(d) > delta) {
+                    l = wc * (2.f * delta * fabsf(d) - delta * delta);
+                    g = 2.f * wc * copysignf(delta, d) * inv_count;
+                } else {
+                    l = wc * d * d;
+                    g = 2.f * wc * d * inv_count;
+                }
             }
         }
+        if (project) {
+            // the 16 channels of one sample are 16 consecutive lanes
+            float s = g;
+            for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, 16);
+            if (c < cv) g -= s / (float)cv;
+        }
+        if (in_range) dout[i] = __float2bfloat16(g);
+        lsum += l;
     }
-    if (project) {
-        // the 16 channels of one sample are 16 consecutive lanes
-        float s = g;
-        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, 16);
-        if (c < cv) g -= s / (float)cv;
+    // one atomic per CTA (one per warp, 65 536 of them on the one address, was
+    // 90 us of 32 x 4096 samples; 16 us so)
+    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_down_sync(0xffffffffu, lsum, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = lsum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float s = 0.f;
+        for (int w = 0; w < 8; ++w) s += part[w];
+        if (s != 0.f) atomicAdd(loss, s * inv_count);
     }
-    if (in_range) dout[i] = __float2bfloat16(g);
-    // warp sum, one atomic per warp
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0 && l != 0.f) atomicAdd(loss, l * inv_count);
 }
 
 // Adam (Kingma & Ba 2015) on f32 parameters
@@ -1616,6 +1838,25 @@ int32_t launch_wgrad_tc(const __nv_bfloat16* dy, const __nv_bfloat16* x, float* 
     return cudaGetLastError() == cudaSuccess ? EEMD_SG_OK : EEMD_SG_E_CUDA;
 }
 
+// the warp-specialised form: one CTA per SM, operands through tensor maps
+template <int CX, int NY>
+int32_t launch_wgrad_ws(const void* dy, const void* x, float* dw, float* db, int B, int T, int nv, int cv, int dil,
+                        int* err, long long spin, cudaStream_t st) {
+    using G = WgGeo<CX, NY>;
+    if (cudaFuncSetAttribute(k_wgrad_ws<CX, NY>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM) != cudaSuccess)
+        return EEMD_SG_E_CUDA;
+    CUtensorMap mx, my;
+    int rc = tensor_map3(&mx, x, B, T, CX, CX, CX == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B);
+    if (rc) return rc;
+    rc = tensor_map3(&my, dy, B, T, NY, NY, NY == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B);
+    if (rc) return rc;
+    const long long tiles = (long long)B * ((T + G::KT - 1) / G::KT);
+    const int grid = (int)(tiles < 148 ? tiles : 148);
+    if (grid < 1) return EEMD_SG_OK;
+    k_wgrad_ws<CX, NY><<<grid, WG_THREADS, G::SMEM, st>>>(mx, my, dw, db, B, T, nv, cv, dil, err, spin);
+    return cudaGetLastError() == cudaSuccess ? EEMD_SG_OK : EEMD_SG_E_CUDA;
+}
+
 extern "C" {
 
 int32_t eemd_sg_version(void) { return EEMD_SG_ABI_VERSION; }
@@ -1682,6 +1923,14 @@ int32_t eemd_sg_wgrad(const void* dy, const void* x, float* dw, float* db, int32
         const cudaStream_t st = static_cast<cudaStream_t>(stream);
         const auto* pdy = static_cast<const __nv_bfloat16*>(dy);
         const auto* px = static_cast<const __nv_bfloat16*>(x);
+        // whole samples of 32 or 128 bytes at 16-byte aligned addresses go through tensor maps
+        if ((c == 16 || c == 64) && B > 0 && T > 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
+            if (c == 64)
+                return n_rows == 64 ? launch_wgrad_ws<64, 64>(dy, x, dw, db, B, T, nv, cv, dil, err, spin, st)
+                                    : launch_wgrad_ws<64, 16>(dy, x, dw, db, B, T, nv, cv, dil, err, spin, st);
+            return n_rows == 64 ? launch_wgrad_ws<16, 64>(dy, x, dw, db, B, T, nv, cv, dil, err, spin, st)
+                                : launch_wgrad_ws<16, 16>(dy, x, dw, db, B, T, nv, cv, dil, err, spin, st);
+        }
         if (3 * c <= 128)
             return n_rows == 64 ? launch_wgrad_tc<1, 64>(pdy, px, dw, db, B, T, n_rows, c, nv, cv, dil, err, spin, st)
                                 : launch_wgrad_tc<1, 16>(pdy, px, dw, db, B, T, n_rows, c, nv, cv, dil, err, spin, st);
@@ -1702,7 +1951,8 @@ int32_t eemd_sg_loss(const void* out, const void* base, const void* target, void
         return EEMD_SG_E_BADARG;
     const long long n = (long long)B * T * c;
     const float inv = 1.f / (float)((long long)B * (T - 2 * margin) * cv);
-    k_loss<<<(unsigned)((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    const long long blocks = (n + 255) / 256;
+    k_loss<<<(unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(base),
         static_cast<const __nv_bfloat16*>(target), static_cast<__nv_bfloat16*>(dout), loss, B, T, c, cv, margin,
         inv, project, delta, channel_weight);
