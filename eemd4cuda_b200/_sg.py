@@ -12,7 +12,8 @@ SG_E_TIMEOUT = -4
 SG_E_CUDA = -5
 ABI_VERSION = 2
 EXPORTS = ("eemd_sg_version", "eemd_sg_conv", "eemd_sg_pack", "eemd_sg_wgrad", "eemd_sg_loss", "eemd_sg_adam",
-           "eemd_sg_bias", "eemd_sg_scale", "eemd_sg_prepare", "eemd_sg_combine", "eemd_sg_stat_count")
+           "eemd_sg_bias", "eemd_sg_scale", "eemd_sg_prepare", "eemd_sg_combine", "eemd_sg_stat_count",
+           "eemd_sg_pack_layers")
 
 _lib = None
 
@@ -42,6 +43,7 @@ def load() -> ctypes.CDLL:
                                  c_int32, c_int32, c_int32, c_void_p, c_int32, c_void_p, c_int64, c_void_p]
     lib.eemd_sg_pack.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32,
                                  c_void_p]
+    lib.eemd_sg_pack_layers.argtypes = [c_void_p, c_int32, c_void_p]
     lib.eemd_sg_bias.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p]
     lib.eemd_sg_scale.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_void_p]
     lib.eemd_sg_prepare.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -85,6 +87,15 @@ def conv(x, wpk, bias, y, B, T, cin, cout, dil, direction=1, relu=False, mask=No
 def pack(w, wpk, n_rows, c, nv, cv, transpose=False, project=False):
     _check(load().eemd_sg_pack(_p(w), _p(wpk), n_rows, c, nv, cv, int(transpose), int(project), _stream()),
            "eemd_sg_pack")
+
+
+def pack_layers(layers):
+    """Every operand of a network in one launch: per layer (w, b, forward
+    operand, input-gradient operand, padded bias, n_rows, c, nv, cv, project)."""
+    row = []
+    for w, b, wp, wt, bias_, *shape in layers:
+        row += [w.data_ptr(), b.data_ptr(), wp.data_ptr(), wt.data_ptr(), bias_.data_ptr(), *map(int, shape)]
+    _check(load().eemd_sg_pack_layers((c_int64 * len(row))(*row), len(layers), _stream()), "eemd_sg_pack_layers")
 
 
 def bias(b, out, n_rows, nv, project=False):

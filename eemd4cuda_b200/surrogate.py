@@ -180,12 +180,8 @@ class Net:
 
     def pack(self):
         """bf16 operands (forward and transposed) and the padded bias from the master weights."""
-        for lay in self.layers:
-            SG.pack(lay["w"], lay["wp"], lay["cout_p"], lay["cin_p"], lay["cout_v"], lay["cin_v"],
-                    project=lay["project"])
-            SG.pack(lay["w"], lay["wt"], lay["cin_p"], lay["cout_p"], lay["cin_v"], lay["cout_v"], transpose=True,
-                    project=lay["project"])
-            SG.bias(lay["b"], lay["bias"], lay["cout_p"], lay["cout_v"], project=lay["project"])
+        SG.pack_layers([(lay["w"], lay["b"], lay["wp"], lay["wt"], lay["bias"], lay["cout_p"], lay["cin_p"],
+                         lay["cout_v"], lay["cin_v"], lay["project"]) for lay in self.layers])
 
     def layer(self, i, src, dst, B, T, tensor_cores=True):
         lay = self.layers[i]

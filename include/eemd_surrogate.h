@@ -62,6 +62,12 @@ int32_t eemd_sg_pack(const float* w, void* w_packed, int32_t n_rows, int32_t c, 
  * nv <= n < n_rows (n_rows <= 1024). */
 int32_t eemd_sg_bias(const float* b, float* bias, int32_t n_rows, int32_t nv, int32_t project, void* stream);
 
+/* eemd_sg_pack (both operands) and eemd_sg_bias of up to 16 layers in one
+ * launch.  table (host, read during the call): 10 values per layer, the device
+ * addresses of w [nv][3][cv], b, the forward operand, the input-gradient operand
+ * and the padded bias, then n_rows, c, nv, cv and project. */
+int32_t eemd_sg_pack_layers(const int64_t* table, int32_t n_layers, void* stream);
+
 /* Accumulates dw[n][tap][c] += sum_t dy[b][t][n] * x[b][t+(tap-1)*dil][c]
  * (n < nv, c < cv) and db[n] += sum_t dy[b][t][n]; dy is [B][T][n_rows],
  * x is [B][T][c] (both bf16, n_rows, c <= 64).  tensor_cores != 0 (and n_rows

@@ -56,3 +56,24 @@ def test_loss_sums(B, T):
     assert abs(float(acc.item()) - np.sum(d * d) / count) <= 1e-5 * np.sum(d * d) / count
     g = 2.0 * d / count
     assert np.max(np.abs(dout.double().cpu().numpy() - g)) <= 2 ** -8 * np.max(np.abs(g))
+
+
+@pytest.mark.parametrize("project", [False, True])
+def test_pack_layers_equals_pack_and_bias(project):
+    """One launch for every layer gives each layer's own eemd_sg_pack (both
+    operands) and eemd_sg_bias, bit for bit, padded channel counts included."""
+    g = torch.Generator().manual_seed(1)
+    layers, want = [], []
+    for N, C, nv, cv in [(64, 16, 64, 11), (64, 64, 64, 64), (16, 64, 6, 64), (16, 16, 10, 16)]:
+        w, b = torch.randn((nv, 3, cv), generator=g).cuda(), torch.randn((nv,), generator=g).cuda()
+        outs = [[torch.full((N * 3 * C,), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+                + [torch.full((N,), 7.0, device="cuda")] for _ in range(2)]
+        layers.append((w, b, *outs[0], N, C, nv, cv, project))
+        _sg.pack(w, outs[1][0], N, C, nv, cv, project=project)
+        _sg.pack(w, outs[1][1], C, N, cv, nv, transpose=True, project=project)
+        _sg.bias(b, outs[1][2], N, nv, project=project)
+        want.append(outs)
+    _sg.pack_layers(layers)
+    torch.cuda.synchronize()
+    for got, ref in want:
+        assert all(torch.equal(u, v) for u, v in zip(got, ref))
