@@ -43,6 +43,15 @@ __device__ __forceinline__ void raise(int* err, int code) {
     if (err) atomicCAS(err, 0, code);
 }
 
+// Kernels launched with launch_after may start while the stream's previous
+// kernel drains (programmatic dependent launch: its own start-up then overlaps
+// that kernel's tail); they wait here before their first access to memory that
+// it may have written or still reads.
+__device__ __forceinline__ void after_previous_kernel() {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -745,16 +754,6 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant
     const uint32_t b_base = a_base + NS * G::A_BYTES;
     const uint32_t o_base = b_base + G::B_BYTES;
     unsigned char* const so = sm + NS * G::A_BYTES + G::B_BYTES;
-    for (int i = tid; i < COUT; i += WS_THREADS) sbias[i] = bias ? bias[i] : 0.f;
-    // weights: the packed K-major image (8-element chunks (n, k8) at k8*COUT*8 + (n/8)*64 + (n%8)*8)
-    // into swizzled rows: tap k8 / KC, row n, chunk k8 % KC
-    for (int i = tid; i < COUT * 3 * KC; i += WS_THREADS) {
-        const int n = i % COUT, k8 = i / COUT;
-        const int tap = k8 / KC, c8 = k8 % KC;
-        const uint4 v = *reinterpret_cast<const uint4*>(wpk + (size_t)k8 * COUT * 8 + (n >> 3) * 64 + (n & 7) * 8);
-        *reinterpret_cast<uint4*>(sm + NS * G::A_BYTES + tap * G::B_TAP + (n >> 3) * G::SBO + (n & 7) * G::ROWB +
-                                  (G::chunk(c8, n) << 4)) = v;
-    }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                          smem_u32(&tmem_slot)),
@@ -772,6 +771,17 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant
         }
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    after_previous_kernel();
+    for (int i = tid; i < COUT; i += WS_THREADS) sbias[i] = bias ? bias[i] : 0.f;
+    // weights: the packed K-major image (8-element chunks (n, k8) at k8*COUT*8 + (n/8)*64 + (n%8)*8)
+    // into swizzled rows: tap k8 / KC, row n, chunk k8 % KC
+    for (int i = tid; i < COUT * 3 * KC; i += WS_THREADS) {
+        const int n = i % COUT, k8 = i / COUT;
+        const int tap = k8 / KC, c8 = k8 % KC;
+        const uint4 v = *reinterpret_cast<const uint4*>(wpk + (size_t)k8 * COUT * 8 + (n >> 3) * 64 + (n & 7) * 8);
+        *reinterpret_cast<uint4*>(sm + NS * G::A_BYTES + tap * G::B_TAP + (n >> 3) * G::SBO + (n & 7) * G::ROWB +
+                                  (G::chunk(c8, n) << 4)) = v;
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the weights, for the MMA
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -999,6 +1009,7 @@ struct PackTable {
 };
 
 __global__ void __launch_bounds__(256) k_pack_layers(const __grid_constant__ PackTable P) {
+    after_previous_kernel();
     int q = 0;
     while (q + 1 < P.n && (int)blockIdx.x >= P.l[q + 1].first) ++q;
     const PackLayer& L = P.l[q];
@@ -1286,6 +1297,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constan
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    after_previous_kernel();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -1430,6 +1442,7 @@ __global__ void k_loss(const __nv_bfloat16* __restrict__ out, const __nv_bfloat1
                        int C, int cv, int margin, float inv_count, int project, float delta,
                        const float* __restrict__ wch) {
     __shared__ float part[8];
+    after_previous_kernel();
     const long long n = (long long)B * T * C;
     float lsum = 0.f;
     // (every lane of a warp takes part in each turn: the projection's shuffles)
@@ -1481,6 +1494,7 @@ __global__ void k_loss(const __nv_bfloat16* __restrict__ out, const __nv_bfloat1
 // whose gradient norm is not finite is skipped)
 __global__ void k_adam(float* p, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
                        float bc1, float bc2, const float* gnorm2, float max_norm) {
+    after_previous_kernel();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float sc = 1.f;
@@ -1500,6 +1514,7 @@ __global__ void k_adam(float* p, const float* g, float* m, float* v, int n, floa
 // out[0] = sum of g[i]^2 (one CTA, fixed order)
 __global__ void __launch_bounds__(1024) k_sumsq(const float* __restrict__ g, int n, float* out) {
     __shared__ float part[32];
+    after_previous_kernel();
     float a = 0.f;
     for (int i = threadIdx.x; i < n; i += 1024) a = fmaf(g[i], g[i], a);
     for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
@@ -1697,6 +1712,23 @@ __global__ void k_gate(const double* __restrict__ partial, int S, int chunks, in
 using namespace sg;
 
 namespace {
+// a launch that may begin while the stream's previous kernel drains (the
+// kernel calls after_previous_kernel)
+template <typename... Params, typename... Args>
+void launch_after(void (*fn)(Params...), int grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);  // (the caller reads the last error)
+}
+
 // 3-D tensor map of the input [B][T][CIN] bf16 with the box {8, 128, 1}
 using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1789,9 +1821,8 @@ int launch_ws(const void* in, const void* wpk, const float* bias, void* out, int
     }
     const int tiles = B * ((T + TM - 1) / TM);
     const int grid = tiles < sms ? tiles : sms;
-    k_conv_ws<CIN, COUT><<<grid, WS_THREADS, G::SMEM, st>>>(mi, mo, static_cast<const __nv_bfloat16*>(wpk), bias,
-                                                           B, T, dil, dir, relu,
-                                                           static_cast<const __nv_bfloat16*>(mask), err, spin);
+    launch_after(k_conv_ws<CIN, COUT>, grid, WS_THREADS, G::SMEM, st, mi, mo, static_cast<const __nv_bfloat16*>(wpk),
+                 bias, B, T, dil, dir, relu, static_cast<const __nv_bfloat16*>(mask), err, spin);
     return cudaGetLastError() == cudaSuccess ? EEMD_SG_OK : EEMD_SG_E_CUDA;
 }
 
@@ -1889,7 +1920,7 @@ int32_t launch_wgrad_ws(const void* dy, const void* x, float* dw, float* db, int
     const long long tiles = (long long)B * ((T + G::KT - 1) / G::KT);
     const int grid = (int)(tiles < 148 ? tiles : 148);
     if (grid < 1) return EEMD_SG_OK;
-    k_wgrad_ws<CX, NY><<<grid, WG_THREADS, G::SMEM, st>>>(mx, my, dw, db, B, T, nv, cv, dil, err, spin);
+    launch_after(k_wgrad_ws<CX, NY>, grid, WG_THREADS, G::SMEM, st, mx, my, dw, db, B, T, nv, cv, dil, err, spin);
     return cudaGetLastError() == cudaSuccess ? EEMD_SG_OK : EEMD_SG_E_CUDA;
 }
 
@@ -1976,7 +2007,7 @@ int32_t eemd_sg_pack_layers(const int64_t* table, int32_t n_layers, void* stream
         L.first = ctas;
         ctas += (2 * L.N * 3 * L.C + L.N + 255) / 256;
     }
-    k_pack_layers<<<ctas, 256, 0, static_cast<cudaStream_t>(stream)>>>(P);
+    launch_after(k_pack_layers, ctas, 256, 0, static_cast<cudaStream_t>(stream), P);
     return cudaGetLastError() == cudaSuccess ? EEMD_SG_OK : EEMD_SG_E_CUDA;
 }
 
@@ -2018,7 +2049,7 @@ int32_t eemd_sg_loss(const void* out, const void* base, const void* target, void
     const long long n = (long long)B * T * c;
     const float inv = 1.f / (float)((long long)B * (T - 2 * margin) * cv);
     const long long blocks = (n + 255) / 256;
-    k_loss<<<(unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_after(k_loss, (int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, static_cast<cudaStream_t>(stream),
         static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(base),
         static_cast<const __nv_bfloat16*>(target), static_cast<__nv_bfloat16*>(dout), loss, B, T, c, cv, margin,
         inv, project, delta, channel_weight);
@@ -2030,9 +2061,9 @@ int32_t eemd_sg_adam(float* p, const float* g, float* m, float* v, int32_t n, fl
     if (!p || !g || !m || !v || n < 0 || step < 1 || (max_norm > 0.f && !work)) return EEMD_SG_E_BADARG;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
-    if (max_norm > 0.f) k_sumsq<<<1, 1024, 0, st>>>(g, n, work);
-    k_adam<<<(n + 255) / 256, 256, 0, st>>>(p, g, m, v, n, lr, b1, b2, eps, bc1, bc2,
-                                            max_norm > 0.f ? work : nullptr, max_norm);
+    if (max_norm > 0.f) launch_after(k_sumsq, 1, 1024, 0, st, g, n, work);
+    launch_after(k_adam, (n + 255) / 256, 256, 0, st, p, g, m, v, n, lr, b1, b2, eps, bc1, bc2,
+                                            max_norm > 0.f ? work : static_cast<float*>(nullptr), max_norm);
     return cudaGetLastError() == cudaSuccess ? EEMD_SG_OK : EEMD_SG_E_CUDA;
 }
 
