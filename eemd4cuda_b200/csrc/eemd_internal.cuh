@@ -76,9 +76,9 @@ struct Header {
 
 struct TaskDesc {
     int64_t x_off;      // element offset of the task's source signal in x
-    int64_t s_off;      // element offset in the residual array (and resid_out)
-    int64_t imf_off;    // element offset of IMF slot 0 (slot m at + m*n)
-    int64_t noise_off;  // element offset in the injected noise array
+    int64_t s_off;      // element offset in the residual array
+    int64_t imf_off;    // element offset of IMF slot 0 (slot m at + m rows, padded in the workspace)
+    int64_t noise_off;  // element offset in the injected noise array (and resid_out)
     int32_t n;          // samples
     int32_t signal;
     int32_t trial;      // absolute trial index (Philox counter)
@@ -114,11 +114,13 @@ struct Ctx {
                                   //   of four (fast: the monomial of interval [k, k+1]; exact: y_k,
                                   //   M_k), then the knots' sample indices [2 env][kcap]
     void* w1;                     // per slot: scratch h buffer [slot_n] (storage type)
+    void* w0;                     // per slot: a second scratch h buffer, or null
     void* r1;                     // per slot: second residual buffer [slot_n] (storage type)
     uint32_t* ri;                 // per slot: run records [2 parity][slot_runs]
     double2* scr;                 // exact-mode solve scratch: [rows][grid threads]
     const void* x;
     const void* noise;
+    void* resid_out;              // optional: final residuals [task][n] (dtype)
     int32_t* knot_log;            // optional [task][max_imf][max_sifts][2]
     int32_t* mode_sifts;          // optional [task][max_imf]
     int64_t slot_knots;           // kt/ky elements per slot
@@ -131,6 +133,7 @@ struct Ctx {
     int32_t max_sifts, max_imf, min_extrema, end_mode, rules, noise_mode;
     int32_t B, S, scr_rows;
     int32_t nw;                   // warps per CTA of this launch
+    int32_t imf_pad;              // IMF rows start on 32 bytes (rows of the workspace)
     double tau;
     double noise_scale;           // EEMD_NOISE_SCALED: the factor on noise[task][n]
     uint64_t seed;

@@ -83,3 +83,81 @@ def test_clipped_intervals(end, dtype, csize):
     cfg = M.EngineConfig(cluster_size=csize, cta_warps=4)
     check(end_rows(), 1e-9 if dtype == np.float64 else 1e-5, max_sifts=1, max_imf=1, end=end, dtype=dtype,
           config=cfg)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n", [1000, 1001, 1003, 4099])
+def test_row_alignment_changes_nothing(dtype, n):
+    """The caller's IMF rows on and off the 32-byte grid (sifted in a second
+    scratch there), rows of the workspace padded to it, and the unpadded rows
+    of a workspace of the bare size: the same IMFs and residuals bit for bit."""
+    torch = pytest.importorskip("torch")
+    from eemd4cuda_b200 import _lib as L
+
+    E, M_ = 3, 4
+    x = np.concatenate(rows_of([n], n) * E) + 0.1 * np.random.default_rng(n).standard_normal(E * n)
+    xd = torch.from_numpy(x.astype(dtype)).cuda()
+    p = M.make_params(dtype=dtype, noise_mode=L.EEMD_NOISE_PREPERTURBED, tau=0.25, max_sifts=9, max_imf=M_)
+    tdt = torch.float32 if dtype == np.float32 else torch.float64
+    got = []
+    for shift in (0, 1):
+        buf = torch.zeros((E * M_ * n + 8,), dtype=tdt, device="cuda")
+        res = torch.zeros((E * n,), dtype=tdt, device="cuda")
+        imfs = buf[shift:shift + E * M_ * n]
+        ws = torch.empty((L.workspace_size(p, [n], E, True),), dtype=torch.uint8, device="cuda")
+        L.run(p, xd, [n], 0, E, ws, imfs=imfs, resid_out=res)
+        got.append((imfs.clone(), res))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    # one trial at a time through the workspace's own rows: the sum of one is the trial's IMF
+    need = L.workspace_size(p, [n], 1, False)
+    for small in (False, True):
+        for e in range(E):
+            s = torch.zeros((M_ * n,), dtype=torch.float64, device="cuda")
+            c = torch.zeros((M_,), dtype=torch.int32, device="cuda")
+            size = need
+            if small:  # the least workspace that is not refused
+                lo, hi = 0, need
+                while hi - lo > 1:
+                    mid = (lo + hi) // 2
+                    try:
+                        L.run(p, xd[e * n:(e + 1) * n], [n], 0, 1, torch.empty((mid,), dtype=torch.uint8, device="cuda"))
+                        hi = mid
+                    except L.EngineError as err:
+                        assert err.status == L.EEMD_E_NOMEM
+                        lo = mid
+                size = hi
+            ws = torch.empty((size,), dtype=torch.uint8, device="cuda")
+            L.run(p, xd[e * n:(e + 1) * n], [n], 0, 1, ws, imf_sum=s, mode_count=c)
+            want = got[0][0].view(E, M_, n)[e].double()
+            assert torch.equal(s.view(M_, n), want * (c > 0)[:, None])
+
+
+@pytest.mark.parametrize("E", [1, 7, 8, 9, 17, 300])
+def test_ensemble_sum_in_trial_order(E):
+    """imf_sum adds the trials that reached a mode in trial order, rounding
+    for rounding, whether all did (the first modes) or only some (the last);
+    it adds to what the caller's array holds."""
+    torch = pytest.importorskip("torch")
+    from eemd4cuda_b200 import _lib as L
+
+    n, M_ = 200, 9
+    x = torch.from_numpy(rows_of([n], 3)[0]).cuda()
+    p = M.make_params(noise_mode=L.EEMD_NOISE_PHILOX, eps=0.5, seed=E, tau=0.25, max_sifts=20, max_imf=M_)
+    imfs = torch.zeros((E, M_, n), dtype=torch.float64, device="cuda")
+    s = torch.full((M_, n), 0.125, dtype=torch.float64, device="cuda")
+    c = torch.full((M_,), 5, dtype=torch.int32, device="cuda")
+    nm = torch.zeros((E,), dtype=torch.int32, device="cuda")
+    ws = torch.empty((L.workspace_size(p, [n], E, True),), dtype=torch.uint8, device="cuda")
+    L.run(p, x, [n], 0, E, ws, imfs=imfs, imf_sum=s, mode_count=c, nmode=nm)
+    h, nm = imfs.cpu().numpy(), nm.cpu().numpy()
+    for m in range(M_):
+        on = [e for e in range(E) if nm[e] > m]
+        assert int(c[m]) == 5 + len(on)
+        want = np.full(n, 0.125)
+        if on:
+            acc = h[on[0], m].copy()
+            for e in on[1:]:
+                acc = acc + h[e, m]
+            want = want + acc
+        assert np.array_equal(s[m].cpu().numpy(), want), m
+    assert E < 300 or len(set(nm)) > 1  # both branches have run
