@@ -30,9 +30,16 @@ import numpy as np
 
 TABLE_DIR = Path(__file__).resolve().parent / "tuning"
 # 49152: about a second of 48 kHz audio, the audio stage's usual segment
-BUCKETS = (4096, 8192, 16384, 32768, 49152, 65536, 262144, 1 << 20, 1 << 22)
-TASKS = (1, 8, 32, 64, 100, 256, 1024, 4096)
-CANDIDATES = (1, 2, 3, 4, 5, 6, 8, 12, 16)   # CTAs per task
+BUCKETS = (2048, 4096, 8192, 16384, 32768, 49152, 65536, 131072, 262144, 1 << 20, 1 << 22)
+TASKS = (1, 4, 8, 16, 32, 48, 64, 100, 128, 192, 256, 512, 1024, 4096)
+CANDIDATES = (1, 2, 3, 4, 5, 6, 8, 10, 12, 16)   # CTAs per task
+# samples per CTA: no fewer are measured (a step of few short signals is a chain
+# of latencies that more CTAs shorten: one 8192-sample EMD runs 0.148 ms on 16
+# CTAs of 4 warps against 0.211 on 4 of 5), and no fewer than SHARE, or than the
+# chosen entry was measured with, are given to a launch's shortest signal
+SMS = 148
+GRAIN = 512
+SHARE = 2048
 WARPS = (4, 5)                                # warps per CTA
 MAX_SAMPLES = 1 << 29  # tasks x length per measurement (workspace and time bound)
 
@@ -51,17 +58,26 @@ def _table(dtype: str):
             for e in d["entries"]]
 
 
-def launch_shape(n_ref: int, n_tasks: int, dtype: str, n_min: int | None = None) -> tuple:
+def launch_shape(n_ref: int, n_tasks: int, dtype: str, n_min: int | None = None, n_max: int | None = None,
+                 total: int | None = None) -> tuple:
     """Tuned (CTAs per task, warps per CTA) for a launch of n_tasks tasks
     whose signals have a median length of n_ref samples and a shortest one
     of n_min (default n_ref): the nearest entry in log length, then in log
     task count, with no more CTAs than give the shortest signal 2048 samples
-    each; (0, 0) when the table has no entry for that storage type."""
+    each, or as few as the entry itself was measured with; (0, 0) when the
+    table has no entry for that storage type.
+
+    An uneven launch (n_max samples in its longest signal, `total` over all
+    tasks) takes enough CTAs that the longest task's share of one is at most
+    1.5 times the samples per CTA slot: the queue hands the longest out first,
+    and one that outlasts the rest is the launch's tail (30 signals of 4096 to
+    262 144 samples x 32 trials: 66 ms on 1 CTA per task, the median length's
+    entry, 42 on 2, 45 on 3)."""
     tab = _table(dtype)
     if not tab:
         return 0, 0
     n_min = n_ref if n_min is None else n_min
-    key = (id(tab), int(n_ref), int(n_tasks), int(n_min))
+    key = (id(tab), int(n_ref), int(n_tasks), int(n_min), n_max, total)
     hit = _SHAPES.get(key)
     if hit is not None:
         return hit
@@ -69,8 +85,17 @@ def launch_shape(n_ref: int, n_tasks: int, dtype: str, n_min: int | None = None)
     bn = min(lengths, key=lambda n: abs(math.log(n) - math.log(max(n_ref, 1))))
     rows = [(t, c, w) for n, t, c, w in tab if n == bn]
     t, c, w = min(rows, key=lambda r: abs(math.log(r[0]) - math.log(max(n_tasks, 1))))
-    # a cluster needs at least 2048 samples per CTA (the engine's own bound)
-    while c > 1 and n_min // c < 2048:
+    # an entry whose tasks all ran at once, for a few more tasks than fit at once,
+    # would run the rest in a second round (twice the time): the next larger entry
+    slots = SMS * (3 if dtype == "f64" or w == 5 else 4)
+    fit = slots // c
+    larger = [r for r in rows if r[0] >= n_tasks]
+    if t <= fit < n_tasks and larger:
+        t, c, w = min(larger)
+    least = min(SHARE, bn // c)
+    if n_max and total and n_max > 2 * n_ref:
+        c = max(c, min(CANDIDATES[-1], math.ceil(n_max * slots / (1.5 * total))))
+    while c > 1 and n_min // c < least:
         c -= 1
     if len(_SHAPES) > 4096:
         _SHAPES.clear()
@@ -86,6 +111,13 @@ def cluster_size(n_min: int, n_tasks: int, dtype: str) -> int:
     return launch_shape(n_min, n_tasks, dtype)[0]
 
 
+@lru_cache(maxsize=1)
+def _signal(n: int):
+    from . import signals
+
+    return signals.harmonic_clicks(n, seed=1)
+
+
 def _measure(n: int, tasks: int, dtype: str, c: int, reps: int, nw: int = 4) -> float:
     """ms of the persistent kernel for `tasks` trials of one n-sample signal
     (2 IMFs x 5 fixed sifts, Philox noise) with clusters of c CTAs of nw warps."""
@@ -93,10 +125,9 @@ def _measure(n: int, tasks: int, dtype: str, c: int, reps: int, nw: int = 4) -> 
 
     from . import _lib as L
     from . import emd_par as M
-    from . import signals
 
     dt = np.float32 if dtype == "f32" else np.float64
-    x = signals.harmonic_clicks(n, seed=1).astype(dt)
+    x = _signal(n).astype(dt)
     p = M.make_params(dtype=dt, noise_mode=L.EEMD_NOISE_PHILOX, eps=0.2, seed=1, tau=0.0, max_sifts=5,
                       max_imf=2, config=M.EngineConfig(cluster_size=c, cta_warps=nw))
     dev = torch.device("cuda", torch.cuda.current_device())
@@ -112,10 +143,10 @@ def _measure(n: int, tasks: int, dtype: str, c: int, reps: int, nw: int = 4) -> 
     return best
 
 
-def tune(dtype: str = "f32", quick: bool = False, reps: int = 2, buckets=None) -> dict:
+def tune(dtype: str = "f32", quick: bool = False, reps: int = 3, buckets=None) -> dict:
     import torch
 
-    buckets = tuple(buckets) if buckets else (BUCKETS[:4] if quick else BUCKETS)
+    buckets = tuple(buckets) if buckets else (BUCKETS[1:5] if quick else BUCKETS)
     entries = []
     for n in buckets:
         for tasks in TASKS:
@@ -124,7 +155,7 @@ def tune(dtype: str = "f32", quick: bool = False, reps: int = 2, buckets=None) -
             times = {}
             for nw in WARPS:
                 for c in CANDIDATES:
-                    if n // c < 2048 and c > 1:
+                    if n // c < GRAIN and c > 1:
                         continue
                     try:
                         times[(nw, c)] = _measure(n, tasks, dtype, c, reps, nw)

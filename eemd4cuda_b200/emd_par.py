@@ -169,10 +169,11 @@ def tuned(p: L.EemdParams, lengths, trial_count: int) -> L.EemdParams:
     if p.cluster_size or p.cta_warps:
         return p
     ls = sorted(int(n) for n in lengths)
-    # an uneven batch is looked up by its median length (most of its work),
-    # with the shortest signal bounding the CTAs per task
+    # an uneven batch is looked up by its median length (most of its work), with
+    # the longest signal's share and the shortest signal bounding the CTAs per task
     c, nw = autotune.launch_shape(ls[len(ls) // 2], len(ls) * int(trial_count),
-                                  "f32" if p.dtype == L.EEMD_F32 else "f64", n_min=ls[0])
+                                  "f32" if p.dtype == L.EEMD_F32 else "f64", n_min=ls[0], n_max=ls[-1],
+                                  total=sum(ls) * int(trial_count))
     if not c:
         return p
     q = L.EemdParams.from_buffer_copy(p)

@@ -161,3 +161,27 @@ def test_ensemble_sum_in_trial_order(E):
             want = want + acc
         assert np.array_equal(s[m].cpu().numpy(), want), m
     assert E < 300 or len(set(nm)) > 1  # both branches have run
+
+
+def test_tuned_shapes_give_the_same_imfs():
+    """The table's launch shapes for a few short signals (up to 16 CTAs of 512
+    samples each) and for an uneven batch against one CTA per task: fixed
+    sifts, so the same IMFs bit for bit."""
+    torch = pytest.importorskip("torch")
+    from eemd4cuda_b200 import _lib as L
+
+    for dtype, lengths, E in [(np.float64, [8192], 1), (np.float32, [3001], 3), (np.float32, [600, 2100, 40000], 4)]:
+        rows = rows_of(lengths, 21)
+        xd = torch.from_numpy(np.concatenate(rows).astype(dtype)).cuda()
+        out = []
+        for shape in (None, 1):
+            p = M.make_params(dtype=dtype, noise_mode=L.EEMD_NOISE_PHILOX, seed=4, tau=0.0, max_sifts=4, max_imf=3)
+            if shape is None:
+                p = M.tuned(p, lengths, E)
+            else:
+                p.cluster_size = 1
+            imfs = torch.zeros((3 * E * sum(lengths),), dtype=torch.from_numpy(np.zeros(1, dtype)).dtype, device="cuda")
+            ws = torch.empty((L.workspace_size(p, lengths, E, True),), dtype=torch.uint8, device="cuda")
+            L.run(p, xd, lengths, 0, E, ws, imfs=imfs)
+            out.append(imfs)
+        assert torch.equal(out[0], out[1]), lengths
