@@ -23,7 +23,9 @@
 
 #include <algorithm>
 #include <climits>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <cstdio>
 #include <cstring>
 #include <numeric>
@@ -2060,8 +2062,8 @@ int make_layout(const eemd_params* p, const int64_t* lengths, int n_signals, int
     L.o_hdr = take(sizeof(Header));
     L.o_td = take(sizeof(TaskDesc) * n_tasks);
     L.o_order = take(sizeof(int32_t) * n_tasks);
-    L.o_tout = take(sizeof(TaskOut) * n_tasks);
     L.o_sd = take(sizeof(SignalDesc) * n_signals);
+    L.o_tout = take(sizeof(TaskOut) * n_tasks);  // (what lies before it is uploaded in one copy)
     L.o_sigma = take(sizeof(double) * n_signals);
     L.o_resid = take(bt * L.NS);
     L.o_imfs = imfs_external ? 0 : take(bt * L.NIMF);
@@ -2317,15 +2319,14 @@ int32_t eemd_run_traced(const eemd_params* p, const void* x, const int64_t* leng
     C.seed = p->seed;
     C.watchdog = p->watchdog != 0 ? p->watchdog : (1LL << 24);
 
-    if (cudaMemsetAsync(base + L.o_hdr, 0, sizeof(Header), st) != cudaSuccess) return EEMD_E_CUDA;
-    if (cudaMemcpyAsync(base + L.o_td, L.td.data(), sizeof(TaskDesc) * L.td.size(), cudaMemcpyHostToDevice,
-                        st) != cudaSuccess)
-        return EEMD_E_CUDA;
-    if (cudaMemcpyAsync(base + L.o_order, L.order.data(), sizeof(int32_t) * L.order.size(),
-                        cudaMemcpyHostToDevice, st) != cudaSuccess)
-        return EEMD_E_CUDA;
-    if (cudaMemcpyAsync(base + L.o_sd, L.sd.data(), sizeof(SignalDesc) * L.sd.size(),
-                        cudaMemcpyHostToDevice, st) != cudaSuccess)
+    // the cleared header and the descriptors in one copy (a memset and three copies
+    // of pageable memory each cost the call 5 to 8 us)
+    std::unique_ptr<char[]> up(new (std::nothrow) char[L.o_tout]());
+    if (!up) return EEMD_E_NOMEM;
+    memcpy(up.get() + L.o_td, L.td.data(), sizeof(TaskDesc) * L.td.size());
+    memcpy(up.get() + L.o_order, L.order.data(), sizeof(int32_t) * L.order.size());
+    memcpy(up.get() + L.o_sd, L.sd.data(), sizeof(SignalDesc) * L.sd.size());
+    if (cudaMemcpyAsync(base + L.o_hdr, up.get(), L.o_tout, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return EEMD_E_CUDA;
     if (knot_log) {
         const size_t nb = sizeof(int32_t) * 2 * L.td.size() * (size_t)p->max_imf * p->max_sifts;
@@ -2341,11 +2342,11 @@ int32_t eemd_run_traced(const eemd_params* p, const void* x, const int64_t* leng
     rc = (p->dtype == EEMD_F64)
              ? run_typed<double>(p, L, C, imf_sum, mode_count, nsift, nmode, flags, st, tr)
              : run_typed<float>(p, L, C, imf_sum, mode_count, nsift, nmode, flags, st, tr);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return EEMD_E_CUDA;
+    Header h;
+    const bool ok = cudaMemcpyAsync(&h, C.hdr, sizeof(Header), cudaMemcpyDeviceToHost, st) == cudaSuccess;
+    if (cudaStreamSynchronize(st) != cudaSuccess || !ok) return EEMD_E_CUDA;
     tr.finish();
     if (rc) return rc;
-    Header h;
-    if (cudaMemcpy(&h, C.hdr, sizeof(Header), cudaMemcpyDeviceToHost) != cudaSuccess) return EEMD_E_CUDA;
     if (h.error) return h.error;
     if (h.n_done != C.n_tasks) return EEMD_E_CUDA;
     return EEMD_OK;

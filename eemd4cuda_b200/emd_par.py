@@ -43,7 +43,7 @@ from dataclasses import asdict, dataclass, field
 import numpy as np
 
 from . import _lib as L
-from .hostcopy import copy_into, fresh_copy, prefault
+from .hostcopy import copy_into, prefault
 
 __all__ = ["decompose", "decompose_many", "EMDResult", "make_reference_sweep", "gpu_eemd_full", "EngineConfig"]
 
@@ -237,15 +237,43 @@ def _pinned(torch, shape, dtype):
     return torch.empty(shape, dtype=dtype, pin_memory=True)
 
 
-def _staging(torch, slots, N):
-    """Pinned host buffers for the outputs of one shape (the latest shape only is kept)."""
-    key = (slots, N)
-    if key not in _STAGE:
-        _STAGE.clear()
-        _STAGE[key] = (torch.empty((slots, N), dtype=torch.float64, pin_memory=True),
-                       torch.empty((N,), dtype=torch.float64, pin_memory=True),
-                       torch.empty((1,), dtype=torch.int32, pin_memory=True))
-    return _STAGE[key]
+def _staging(torch):
+    """The shared pinned staging buffer (PINNED_RESULT_BYTES, allocated once)."""
+    if "buf" not in _STAGE:
+        _STAGE["buf"] = torch.empty((PINNED_RESULT_BYTES // 8,), dtype=torch.float64, pin_memory=True)
+    return _STAGE["buf"]
+
+
+def _staged_copies(torch, pairs, futs=()):
+    """dst[...] = src for (host array, contiguous float64 device tensor) pairs
+    of any size: slices cross to the two halves of the pinned staging buffer,
+    and each is copied out on the copy threads while the next one crosses.
+    `futs`: the prefault futures of the host arrays."""
+    with _STAGE_LOCK:  # callers on several threads share the buffer
+        stage = _staging(torch)
+        half, hs = stage.numel() // 2, stage.numpy()
+        for f in futs:
+            f.result()
+        marks = []
+
+        def out(mark):
+            d, a0, a1, ev, b0 = mark
+            ev.synchronize()
+            copy_into(d[a0:a1], hs[b0:b0 + (a1 - a0)])
+
+        for dst, src in pairs:
+            dst, src = dst.reshape(-1), src.reshape(-1)
+            for i0 in range(0, src.numel(), half):
+                i1 = min(src.numel(), i0 + half)
+                b0 = (len(marks) & 1) * half
+                if len(marks) >= 2:  # the half this slice reuses has been copied out
+                    out(marks[-2])
+                stage[b0:b0 + (i1 - i0)].copy_(src[i0:i1], non_blocking=True)
+                ev = torch.cuda.Event()
+                ev.record(torch.cuda.current_stream(src.device))
+                marks.append((dst, i0, i1, ev, b0))
+        for mark in marks[-2:]:
+            out(mark)
 
 
 class Checkpoint:
@@ -344,6 +372,12 @@ def _run_ensemble(x, *, E, eps, tau, max_sifts, max_imf, min_extrema, end, seed,
             mode_count.copy_(torch.from_numpy(state["mode_count"]))
             cnt[:, :first].copy_(torch.from_numpy(state["counters"]))
     ws = None
+    paged = None
+    if slots * N * 8 > PINNED_RESULT_BYTES:
+        # large results: their host arrays are paged in on the copy threads while the device works
+        # (of the rows an open mode count may reach, those it usually does)
+        mh_host, rh_host = np.empty((slots, N), dtype=np.float64), np.empty((N,), dtype=np.float64)
+        paged = prefault([mh_host[:slots if max_imf != -1 else max(1, slots - 8)], rh_host])
     t0 = time.time()
     for b0 in range(first, E, batch):
         b1 = min(E, b0 + batch)
@@ -381,15 +415,11 @@ def _run_ensemble(x, *, E, eps, tau, max_sifts, max_imf, min_extrema, end, seed,
             imfs = h_mean[:n_modes].numpy()
             residual = h_resid.numpy()
     else:
-        with _STAGE_LOCK, nvtx.range("eemd.download"):  # callers on several threads share the buffers
-            h_mean, h_resid, h_n = _staging(torch, slots, N)
-            h_mean.copy_(imf_mean, non_blocking=True)
-            h_resid.copy_(resid, non_blocking=True)
-            h_n.copy_(n_modes_d, non_blocking=True)
-            ch = cnt.cpu()  # synchronises the stream: every copy above has landed
-            n_modes = int(h_n[0])
-            imfs = fresh_copy(h_mean[:n_modes].numpy())
-            residual = h_resid.numpy().copy()
+        with nvtx.range("eemd.download"):
+            n_modes = int(n_modes_d.item())
+            ch = cnt.cpu()
+            imfs, residual = mh_host[:n_modes], rh_host
+            _staged_copies(torch, ((imfs, imf_mean[:n_modes]), (residual, resid)), paged)
     per_trial_sifts, per_trial_modes, flags_all = ch[0].tolist(), ch[1].tolist(), ch[2].tolist()
     if ck is not None:
         ck.remove()
@@ -419,24 +449,22 @@ def _run_single(x, *, tau, max_sifts, max_imf, min_extrema, end, rules, exact, d
     xd = torch.from_numpy(np.ascontiguousarray(x, dtype=dt)).to(dev)
     ws = torch.empty((L.workspace_size(p, [N], 1, True),), dtype=torch.uint8, device=dev)
     # (the engine writes every IMF row it returns; the rows past the mode count are not read)
-    imfs = torch.empty((1, slots, N), dtype=tdt, device=dev)
-    resid = torch.empty((1, N), dtype=tdt, device=dev)
+    # the IMF rows and, behind them, the residual: one copy back
+    rows = torch.empty((slots + 1, N), dtype=tdt, device=dev)
     # the counters in one array (sifts, modes, flags, sifts per mode): one copy back
     cnt = torch.empty((3 + slots,), dtype=torch.int32, device=dev)
     t0 = time.time()
-    L.run(p, xd, [N], 0, 1, ws, imfs=imfs, resid_out=resid, nsift=cnt[0:1], nmode=cnt[1:2],
+    L.run(p, xd, [N], 0, 1, ws, imfs=rows, resid_out=rows[slots], nsift=cnt[0:1], nmode=cnt[1:2],
           mode_sifts=cnt[3:], flags=cnt[2:3])
     # every output into pinned memory, one synchronisation
-    h_imfs, h_res = _pinned(torch, (slots, N), torch.float64), _pinned(torch, (N,), torch.float64)
-    h_cnt = _pinned(torch, (3 + slots,), torch.int32)
-    h_imfs.copy_(imfs[0].to(torch.float64), non_blocking=True)
-    h_res.copy_(resid[0].to(torch.float64), non_blocking=True)
+    h_rows, h_cnt = _pinned(torch, (slots + 1, N), torch.float64), _pinned(torch, (3 + slots,), torch.int32)
+    h_rows.copy_(rows.to(torch.float64), non_blocking=True)
     h_cnt.copy_(cnt, non_blocking=True)
     torch.cuda.current_stream(dev).synchronize()
     c = h_cnt.tolist()
     nm = int(c[1])
-    out = h_imfs[:nm].numpy()
-    res = h_res.numpy()
+    out = h_rows[:nm].numpy()
+    res = h_rows[slots].numpy()
     stats = dict(method="gpu", backend="b200", E=1, n_modes=nm, total_sifts=int(c[0]),
                  per_mode_sifts=[int(v) for v in c[3:3 + nm]], per_trial_total_sifts=np.array([int(c[0])]),
                  max_imf_reached=bool(int(c[2]) & 1 and max_imf == -1),
@@ -580,29 +608,7 @@ def _download(torch, dev, imf_mean, resid, n_modes, paged):
         return h_m.numpy(), h_r.numpy(), h_n.numpy()
     mh, rh, futs = paged
     nh = n_modes.cpu().numpy()
-    with _STAGE_LOCK:
-        stage = _staging(torch, 2, PINNED_RESULT_BYTES // 16)[0].reshape(-1)  # 64 MB, two halves
-        half = stage.numel() // 2
-        for f in futs:
-            f.result()
-        for dst, src in ((mh, imf_mean), (rh, resid)):
-            n, marks, i0 = src.numel(), [], 0
-            hs = stage.numpy()
-            while i0 < n:
-                i1 = min(n, i0 + half)
-                buf = (len(marks) & 1) * half
-                if len(marks) >= 2:  # the half this slice reuses has been copied out
-                    marks[-2][2].synchronize()
-                    a0, a1, _, b0 = marks[-2]
-                    copy_into(dst[a0:a1], hs[b0:b0 + (a1 - a0)])
-                stage[buf:buf + (i1 - i0)].copy_(src[i0:i1], non_blocking=True)
-                ev = torch.cuda.Event()
-                ev.record()
-                marks.append((i0, i1, ev, buf))
-                i0 = i1
-            for a0, a1, ev, b0 in marks[-2:]:
-                ev.synchronize()
-                copy_into(dst[a0:a1], hs[b0:b0 + (a1 - a0)])
+    _staged_copies(torch, ((mh, imf_mean), (rh, resid)), futs)
     return mh, rh, nh
 
 
@@ -631,13 +637,21 @@ def gpu_eemd_full(x, E=64, tau=0.25, max_sifts=50, max_imf=12, seed=0, K=None, n
     p = tuned(p, [N], E)
     xd = torch.from_numpy(np.ascontiguousarray(x)).to(dev)
     out = torch.zeros((E, int(max_imf), N), dtype=torch.float64, device=dev)
-    nsift = torch.zeros((E,), dtype=torch.int32, device=dev)
-    nmode = torch.zeros((E,), dtype=torch.int32, device=dev)
+    cnt = torch.zeros((2, E), dtype=torch.int32, device=dev)
     ws = torch.empty((L.workspace_size(p, [N], E, True),), dtype=torch.uint8, device=dev)
-    L.run(p, xd, [N], 0, E, ws, imfs=out, nsift=nsift, nmode=nmode)
-    nm = nmode.cpu().numpy()
+    L.run(p, xd, [N], 0, E, ws, imfs=out, nsift=cnt[0], nmode=cnt[1])
+    nsift, nm = (a.copy() for a in cnt.cpu().numpy())
     maxm = int(nm.max()) if nm.size else 0
-    return out[:, :maxm].cpu().numpy(), nsift.cpu().numpy(), nm
+    # results as decompose returns them: pinned memory of their own, large ones through the staging
+    if E * maxm * N * 8 <= PINNED_RESULT_BYTES:
+        h = _pinned(torch, (E, maxm, N), torch.float64)
+        h.copy_(out[:, :maxm], non_blocking=True)
+        torch.cuda.current_stream(dev).synchronize()
+        return h.numpy(), nsift, nm
+    imfs = np.empty((E, maxm, N), dtype=np.float64)
+    futs = prefault([imfs])
+    _staged_copies(torch, ((imfs, out[:, :maxm].contiguous()),), futs)
+    return imfs, nsift, nm
 
 
 # =====================================================================
