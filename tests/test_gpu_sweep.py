@@ -85,6 +85,27 @@ def test_clipped_intervals(end, dtype, csize):
           config=cfg)
 
 
+def density_rows():
+    """Float32 runs of 8 samples with one, two, three and four knots, and slow
+    rows in which single runs (at a tile's start, middle and end) have up to
+    eight: tiles on both sides of the sparse store's bound, one next to the other."""
+    n = 1541
+    t = np.arange(n, dtype=float)
+    out = [np.sin(2 * np.pi * (t + 0.3) / p) * (1 + 0.2 * np.cos(t / 97.0)) for p in (16.3, 8.1, 7.9, 5.2, 4.1)]
+    for at in (512, 640, 764, 1019):
+        fast = np.where((t >= at) & (t < at + 9), 1.0, 0.0) * np.cos(np.pi * t) * (1 + 0.01 * (t - at))
+        out.append(np.sin(2 * np.pi * t / 61.7) + fast)
+    return out
+
+
+@pytest.mark.parametrize("end", ["natural", "mirror"])
+def test_knot_densities_float32(end):
+    """Bound as in test_tile_edges_float32; the fast runs' envelopes stay of
+    the order of max|x| as their extrema alternate about the slow one."""
+    cfg = M.EngineConfig(cluster_size=1, cta_warps=4)
+    check(density_rows(), 1e-5, max_sifts=1, max_imf=1, end=end, dtype=np.float32, config=cfg)
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("n", [1000, 1001, 1003, 4099])
 def test_row_alignment_changes_nothing(dtype, n):
