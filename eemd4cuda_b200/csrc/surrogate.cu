@@ -674,11 +674,18 @@ __global__ void __launch_bounds__(32 * EW) k_conv_tma(const __grid_constant__ CU
 //   MMA warp   (lane 0): waits full[s] and the accumulator's release
 //                        (acce[k & 1]), issues the 3 * CIN / 16 MMAs of tile k into
 //                        accumulator k & 1, commits to empty[s] and accf[k & 1];
-//   8 epilogue warps   : read their lane quadrant x half the columns of the
-//                        accumulator, release it, add bias / ReLU / mask,
-//                        write the bf16 tile into a swizzled staging buffer,
-//                        and one thread stores it with a bulk-tensor store
-//                        (rows past T are clipped by the tensor map).
+//   2 groups of 4 epilogue warps, one per accumulator, so that one group's chain
+//                        of latencies runs beside the other's: read their lane
+//                        quadrant, release the accumulator, add bias / ReLU /
+//                        mask (asked for before the accumulator is awaited),
+//                        write the bf16 tile into the group's swizzled staging
+//                        buffer, and one thread stores it with a bulk-tensor
+//                        store (rows past T are clipped by the tensor map).
+// The 8 layers over 16 x 65536 samples: 485 us with all eight warps on each
+// tile, the mask loaded after the wait and the first copies issued after the
+// weights; 467 with those two moved, 458 with the groups (of 300 that its bytes
+// take).  Not the loads: one tap of the three, or 8 stages of one, 450; L2
+// prefetches 457.
 // The MMA's K order (tap-major, 16 channels per instruction) is the same as
 // the other forms', so the results are bit-identical to theirs.  Every wait
 // is bounded; a wait that gives up sets *err and every role leaves its loop.
@@ -714,14 +721,15 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// named barrier 1 over the epilogue warps, OR of v over their threads
-__device__ __forceinline__ bool epi_bar_or(bool v) {
+// named barriers 1 and 2 over an epilogue group's four warps, and the OR of v over its threads
+__device__ __forceinline__ void epi_bar(int grp) { asm volatile("bar.sync %0, 128;\n" ::"r"(grp + 1) : "memory"); }
+__device__ __forceinline__ bool epi_bar_or(int grp, bool v) {
     uint32_t r;
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\t"
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, 128, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}\n"
         : "=r"(r)
-        : "r"((uint32_t)v), "n"(32 * WS_EPI)
+        : "r"((uint32_t)v), "r"(grp + 1)
         : "memory");
     return r != 0;
 }
@@ -739,14 +747,13 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant
     constexpr int KC = CIN / 8;            // 16-byte chunks per operand row
     constexpr int ACOLS = COUT < 32 ? 32 : COUT;
     constexpr int TCOLS = 2 * ACOLS;
-    constexpr int NC = COUT * 4 / WS_EPI;  // accumulator columns per epilogue warp
     constexpr uint32_t IDESC = instr_desc(TM, COUT);
     static_assert((CIN == 64 || CIN == 16) && (COUT == 64 || COUT == 16), "shape");
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[NS], empty[NS], accf[2], acce[2];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
-    __shared__ float sbias[COUT];
+    __shared__ __align__(16) float sbias[COUT];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t a_base = (raw + 1023u) & ~1023u;  // swizzled operands need 1024-byte alignment
@@ -760,19 +767,42 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant
                      "r"(TCOLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
     }
-    if (tid == 0) {
+    if (tid == 32 * WS_EPI) {
         for (int i = 0; i < NS; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&full[i])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&empty[i])));
         }
         for (int i = 0; i < 2; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&accf[i])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&acce[i])), "n"(WS_EPI));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&acce[i])), "n"(WS_EPI / 2));
         }
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    const int tiles_per_b = (T + TM - 1) / TM;
+    const int n_tiles = B * tiles_per_b;
+    const int nk = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    auto load_tile = [&](int k) {  // (the copy thread: tile k's taps into their stage)
+        const int s = k % NS;
+        const int tile = blockIdx.x + k * gridDim.x;
+        const int b = tile / tiles_per_b, t0 = (tile % tiles_per_b) * TM;
+        const uint32_t dst = a_base + s * G::A_BYTES;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(&full[s])),
+                     "n"(G::A_BYTES)
+                     : "memory");
+#pragma unroll
+        for (int tap = 0; tap < 3; ++tap)
+            asm volatile(
+                "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], "
+                "[%1, {%2, %3, %4}], [%5];\n" ::"r"(dst + tap * G::TAP_BYTES),
+                "l"(reinterpret_cast<uint64_t>(&tin)), "r"(0), "r"(t0 + dir * (tap - 1) * dil), "r"(b),
+                "r"(smem_u32(&full[s]))
+                : "memory");
+    };
     after_previous_kernel();
+    // the first stages are on their way while the weights are laid out
+    if (tid == 32 * WS_EPI)
+        for (int k = 0; k < nk && k < NS; ++k) load_tile(k);
     for (int i = tid; i < COUT; i += WS_THREADS) sbias[i] = bias ? bias[i] : 0.f;
     // weights: the packed K-major image (8-element chunks (n, k8) at k8*COUT*8 + (n/8)*64 + (n%8)*8)
     // into swizzled rows: tap k8 / KC, row n, chunk k8 % KC
@@ -788,10 +818,6 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    const int tiles_per_b = (T + TM - 1) / TM;
-    const int n_tiles = B * tiles_per_b;
-    const int nk = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-
     if (warp == WS_EPI) {
         // ---------------- copy warp ----------------
         if (lane == 0) {
@@ -803,22 +829,10 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant
                     abort_flag = 1;
                     break;
                 }
-                const int tile = blockIdx.x + k * gridDim.x;
-                const int b = tile / tiles_per_b, t0 = (tile % tiles_per_b) * TM;
-                const uint32_t dst = a_base + s * G::A_BYTES;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(&full[s])),
-                             "n"(G::A_BYTES)
-                             : "memory");
-#pragma unroll
-                for (int tap = 0; tap < 3; ++tap)
-                    asm volatile(
-                        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], "
-                        "[%1, {%2, %3, %4}], [%5];\n" ::"r"(dst + tap * G::TAP_BYTES),
-                        "l"(reinterpret_cast<uint64_t>(&tin)), "r"(0), "r"(t0 + dir * (tap - 1) * dil), "r"(b),
-                        "r"(smem_u32(&full[s]))
-                        : "memory");
+                if (k >= NS) load_tile(k);
             }
             // copies still in flight (only when a role gave up) land before the CTA leaves
+            k = max(k, min(nk, NS));
             for (int j = k - 1; j >= 0 && j >= k - NS; --j) wait_parity(&full[j % NS], (uint32_t)(j / NS) & 1u, spin_limit);
         }
     } else if (warp == WS_EPI + 1) {
@@ -857,61 +871,75 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant
         }
     } else {
         // ---------------- epilogue warps ----------------
-        const int quad = warp & 3, cb = (warp >> 2) * NC;
+        const int grp = warp >> 2, quad = warp & 3;
         const int r = 32 * quad + lane;  // tile row of this lane
-        for (int k = 0; k < nk; ++k) {
-            const int a = k & 1;
+        const bool leader = (tid & 127) == 0;
+        unsigned char* const ob = so + grp * G::O_BYTES;
+        for (int k = grp; k < nk; k += 2) {
             const int tile = blockIdx.x + k * gridDim.x;
             const int b = tile / tiles_per_b, t0 = (tile % tiles_per_b) * TM;
-            const bool ok = __all_sync(0xffffffffu, wait_parity(&accf[a], (uint32_t)(k >> 1) & 1u, spin_limit));
+            const int t = t0 + r;
+            uint4 mv[COUT / 8];
+            if (mask) {
+#pragma unroll
+                for (int j = 0; j < COUT / 8; ++j) mv[j] = make_uint4(0, 0, 0, 0);
+                if (t < T) {
+#pragma unroll
+                    for (int j = 0; j < COUT / 8; ++j)
+                        mv[j] = *reinterpret_cast<const uint4*>(mask + ((size_t)b * T + t) * COUT + 8 * j);
+                }
+            }
+            const bool ok = __all_sync(0xffffffffu, wait_parity(&accf[grp], (uint32_t)(k >> 1) & 1u, spin_limit));
+            uint32_t o[COUT / 2];
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                float v[NC];
-                tmem_ld_cols<NC>(tmem + a * ACOLS + ((uint32_t)(32 * quad) << 16) + (uint32_t)cb, v);
+                float v[COUT];
+                tmem_ld_cols<COUT>(tmem + grp * ACOLS + ((uint32_t)(32 * quad) << 16), v);
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&acce[a]);
-                const int t = t0 + r;
-                const __nv_bfloat16* mk = (mask && t < T) ? mask + ((size_t)b * T + t) * COUT + cb : nullptr;
-                unsigned char* const ob = so + (k & 1) * G::O_BYTES;
+                if (lane == 0) mbar_arrive(&acce[grp]);
 #pragma unroll
-                for (int j = 0; j < NC / 8; ++j) {
-                    __align__(16) __nv_bfloat16 h[8];
-                    uint4 mv = make_uint4(0, 0, 0, 0);
-                    if (mk) mv = *reinterpret_cast<const uint4*>(mk + 8 * j);
-                    const __nv_bfloat16* mh = reinterpret_cast<const __nv_bfloat16*>(&mv);
+                for (int i = 0; i < COUT; ++i) v[i] += sbias[i];
+                if (relu) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        float x = v[8 * j + i] + sbias[cb + 8 * j + i];
-                        if (relu) x = fmaxf(x, 0.f);
-                        if (mask && !(__bfloat162float(mh[i]) > 0.f)) x = 0.f;
-                        h[i] = __float2bfloat16(x);
-                    }
-                    const int c = (cb >> 3) + j;  // 16-byte chunk of the output row
-                    const int off = COUT == 64 ? r * 128 + ((c ^ (r & 7)) << 4) : r * (COUT * 2) + (c << 4);
-                    *reinterpret_cast<uint4*>(ob + off) = *reinterpret_cast<const uint4*>(h);
+                    for (int i = 0; i < COUT; ++i) v[i] = fmaxf(v[i], 0.f);
                 }
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < COUT / 2; ++i) {
+                    const __nv_bfloat162 p = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                    o[i] = *reinterpret_cast<const uint32_t*>(&p);
+                }
+                if (mask) {
+                    const __nv_bfloat162 z = __float2bfloat162_rn(0.f);
+#pragma unroll
+                    for (int i = 0; i < COUT / 2; ++i)
+                        o[i] &= __hgt2_mask(reinterpret_cast<const __nv_bfloat162*>(mv)[i], z);
+                }
             }
-            // the stores issued so far (tile k-1's) have read their staging buffer
-            // before tile k+1 overwrites it
-            if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
-            __syncwarp();
-            if (epi_bar_or(!ok)) {
-                if (tid == 0) raise(err, EEMD_SG_E_TIMEOUT);
+            // the group's last store has read its staging buffer before it is written again
+            if (leader) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+            if (epi_bar_or(grp, !ok)) {
+                if (leader) raise(err, EEMD_SG_E_TIMEOUT);
                 abort_flag = 1;
                 break;
             }
-            if (tid == 0) {
+#pragma unroll
+            for (int c = 0; c < COUT / 8; ++c) {
+                const int off = COUT == 64 ? r * 128 + ((c ^ (r & 7)) << 4) : r * (COUT * 2) + (c << 4);
+                *reinterpret_cast<uint4*>(ob + off) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+            }
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            epi_bar(grp);
+            if (leader) {
                 asm volatile(
                     "cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];\n" ::"l"(
                         reinterpret_cast<uint64_t>(&tout)),
-                    "r"(0), "r"(t0), "r"(b), "r"(o_base + (k & 1) * G::O_BYTES)
+                    "r"(0), "r"(t0), "r"(b), "r"(o_base + grp * G::O_BYTES)
                     : "memory");
                 asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
             }
         }
-        if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
+        if (leader) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
     }
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -1288,7 +1316,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constan
                      "r"(G::TCOLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
     }
-    if (tid == 0) {
+    if (tid == 32 * WG_SUM) {
         for (int i = 0; i < NS; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&full[i])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&empty[i])), "n"(1 + WG_SUM));
@@ -1297,15 +1325,33 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constan
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    const int tiles_per_b = (T + G::KT - 1) / G::KT;
+    const int n_tiles = B * tiles_per_b;
+    const int nk = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    auto load_tile = [&](int k) {  // (the copy thread: tile k's boxes into their stage)
+        const int s = k % NS;
+        const int tile = blockIdx.x + k * gridDim.x;
+        const int b = tile / tiles_per_b, t0 = (tile % tiles_per_b) * G::KT;
+        const uint32_t dst = base + s * G::STAGE;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(&full[s])),
+                     "n"(G::STAGE)
+                     : "memory");
+#pragma unroll
+        for (int tap = 0; tap < 4; ++tap)  // (the fourth box is dy)
+            asm volatile(
+                "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], "
+                "[%1, {%2, %3, %4}], [%5];\n" ::"r"(dst + tap * G::XB),
+                "l"(tap < 3 ? reinterpret_cast<uint64_t>(&tx) : reinterpret_cast<uint64_t>(&ty)), "r"(0),
+                "r"(tap < 3 ? t0 + (tap - 1) * dil : t0), "r"(b), "r"(smem_u32(&full[s]))
+                : "memory");
+    };
     after_previous_kernel();
+    if (tid == 32 * WG_SUM)
+        for (int k = 0; k < nk && k < NS; ++k) load_tile(k);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    const int tiles_per_b = (T + G::KT - 1) / G::KT;
-    const int n_tiles = B * tiles_per_b;
-    const int nk = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-
     if (warp == WG_SUM) {
         // ---------------- copy warp ----------------
         if (lane == 0) {
@@ -1317,22 +1363,10 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constan
                     abort_flag = 1;
                     break;
                 }
-                const int tile = blockIdx.x + k * gridDim.x;
-                const int b = tile / tiles_per_b, t0 = (tile % tiles_per_b) * G::KT;
-                const uint32_t dst = base + s * G::STAGE;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(&full[s])),
-                             "n"(G::STAGE)
-                             : "memory");
-#pragma unroll
-                for (int tap = 0; tap < 4; ++tap)  // (the fourth box is dy)
-                    asm volatile(
-                        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], "
-                        "[%1, {%2, %3, %4}], [%5];\n" ::"r"(dst + tap * G::XB),
-                        "l"(tap < 3 ? reinterpret_cast<uint64_t>(&tx) : reinterpret_cast<uint64_t>(&ty)), "r"(0),
-                        "r"(tap < 3 ? t0 + (tap - 1) * dil : t0), "r"(b), "r"(smem_u32(&full[s]))
-                        : "memory");
+                if (k >= NS) load_tile(k);
             }
             // copies still in flight (only when a role gave up) land before the CTA leaves
+            k = max(k, min(nk, NS));
             for (int j = k - 1; j >= 0 && j >= k - NS; --j) wait_parity(&full[j % NS], (uint32_t)(j / NS) & 1u, spin_limit);
         }
     } else if (warp == WG_SUM + 1) {
@@ -1445,37 +1479,53 @@ __global__ void k_loss(const __nv_bfloat16* __restrict__ out, const __nv_bfloat1
     after_previous_kernel();
     const long long n = (long long)B * T * C;
     float lsum = 0.f;
+    // four turns' loads at a time: a turn is otherwise one chain of memory latency,
+    // division and shuffles (32 x 4096 samples, seven turns: 15.7 us so)
+    constexpr int U = 4;
+    const long long stride = (long long)gridDim.x * blockDim.x;
     // (every lane of a warp takes part in each turn: the projection's shuffles)
-    for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < n; i0 += (long long)gridDim.x * blockDim.x) {
-        const long long i = i0 + threadIdx.x;
-        const bool in_range = i < n;
-        float l = 0.f, g = 0.f;
-        int c = 0;
-        if (in_range) {
-            const long long row = n <= 0xffffffffLL ? (long long)((uint32_t)i / (uint32_t)C) : i / C;
-            c = (int)(i - row * C);
-            const int t = n <= 0xffffffffLL ? (int)((uint32_t)row % (uint32_t)T) : (int)(row % T);
-            if (c < cv && t >= margin && t < T - margin) {
-                const float d = (base ? __bfloat162float(base[i]) : 0.f) + __bfloat162float(out[i]) -
-                                __bfloat162float(target[i]);
-                const float wc = wch ? wch[c] : 1.f;
-                if (delta > 0.f && fabsf(d) > delta) {
-                    l = wc * (2.f * delta * fabsf(d) - delta * delta);
-                    g = 2.f * wc * copysignf(delta, d) * inv_count;
-                } else {
-                    l = wc * d * d;
-                    g = 2.f * wc * d * inv_count;
+    for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < n; i0 += U * stride) {
+        float d[U], wc[U];
+        int ch[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long i = i0 + u * stride + threadIdx.x;
+            d[u] = wc[u] = 0.f;
+            ch[u] = -1;  // no element, or one outside the loss
+            if (i < n) {
+                const long long row = n <= 0xffffffffLL ? (long long)((uint32_t)i / (uint32_t)C) : i / C;
+                const int c = (int)(i - row * C);
+                const int t = n <= 0xffffffffLL ? (int)((uint32_t)row % (uint32_t)T) : (int)(row % T);
+                if (c < cv) {
+                    ch[u] = c;
+                    if (t >= margin && t < T - margin) {
+                        d[u] = (base ? __bfloat162float(base[i]) : 0.f) + __bfloat162float(out[i]) -
+                               __bfloat162float(target[i]);
+                        wc[u] = wch ? wch[c] : 1.f;
+                    }
                 }
             }
         }
-        if (project) {
-            // the 16 channels of one sample are 16 consecutive lanes
-            float s = g;
-            for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, 16);
-            if (c < cv) g -= s / (float)cv;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long i = i0 + u * stride + threadIdx.x;
+            float l, g;
+            if (delta > 0.f && fabsf(d[u]) > delta) {
+                l = wc[u] * (2.f * delta * fabsf(d[u]) - delta * delta);
+                g = 2.f * wc[u] * copysignf(delta, d[u]) * inv_count;
+            } else {
+                l = wc[u] * d[u] * d[u];
+                g = 2.f * wc[u] * d[u] * inv_count;
+            }
+            if (project) {
+                // the 16 channels of one sample are 16 consecutive lanes
+                float s = g;
+                for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, 16);
+                if (ch[u] >= 0) g -= s / (float)cv;
+            }
+            if (i < n) dout[i] = __float2bfloat16(g);
+            lsum += l;
         }
-        if (in_range) dout[i] = __float2bfloat16(g);
-        lsum += l;
     }
     // one atomic per CTA (one per warp, 65 536 of them on the one address, was
     // 90 us of 32 x 4096 samples; 16 us so)
@@ -1516,6 +1566,7 @@ __global__ void __launch_bounds__(1024) k_sumsq(const float* __restrict__ g, int
     __shared__ float part[32];
     after_previous_kernel();
     float a = 0.f;
+#pragma unroll 16
     for (int i = threadIdx.x; i < n; i += 1024) a = fmaf(g[i], g[i], a);
     for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = a;
