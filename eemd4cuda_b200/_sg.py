@@ -13,7 +13,7 @@ SG_E_CUDA = -5
 ABI_VERSION = 2
 EXPORTS = ("eemd_sg_version", "eemd_sg_conv", "eemd_sg_pack", "eemd_sg_wgrad", "eemd_sg_loss", "eemd_sg_adam",
            "eemd_sg_bias", "eemd_sg_scale", "eemd_sg_prepare", "eemd_sg_combine", "eemd_sg_stat_count",
-           "eemd_sg_pack_layers")
+           "eemd_sg_pack_layers", "eemd_sg_forward_layers", "eemd_sg_backward_layers")
 
 _lib = None
 
@@ -44,6 +44,8 @@ def load() -> ctypes.CDLL:
     lib.eemd_sg_pack.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32,
                                  c_void_p]
     lib.eemd_sg_pack_layers.argtypes = [c_void_p, c_int32, c_void_p]
+    lib.eemd_sg_forward_layers.argtypes = [c_void_p, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p]
+    lib.eemd_sg_backward_layers.argtypes = [c_void_p, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p]
     lib.eemd_sg_bias.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_int32, c_void_p]
     lib.eemd_sg_scale.argtypes = [c_void_p, c_void_p, c_int32, c_int32, c_void_p]
     lib.eemd_sg_prepare.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -96,6 +98,30 @@ def pack_layers(layers):
     for w, b, wp, wt, bias_, *shape in layers:
         row += [w.data_ptr(), b.data_ptr(), wp.data_ptr(), wt.data_ptr(), bias_.data_ptr(), *map(int, shape)]
     _check(load().eemd_sg_pack_layers((c_int64 * len(row))(*row), len(layers), _stream()), "eemd_sg_pack_layers")
+
+
+def _addresses(tensors):
+    return [t.data_ptr() if t is not None else 0 for t in tensors]
+
+
+def forward_layers(layers, B, T, tensor_cores=True, err=None):
+    """The convolutions of a forward pass in one call: per layer (input,
+    operand, bias, output, mask or None, cin, cout, dil, direction, relu)."""
+    row = []
+    for lay in layers:
+        row += _addresses(lay[:5]) + [int(v) for v in lay[5:]]
+    _check(load().eemd_sg_forward_layers((c_int64 * len(row))(*row), len(layers), B, T, int(tensor_cores), _p(err),
+                                         _stream()), "eemd_sg_forward_layers")
+
+
+def backward_layers(layers, B, T, tensor_cores=True, err=None):
+    """The weight and input gradients of a backward pass in one call: per
+    layer (dy, x, dw, db, transposed operand, dx or None, n_rows, c, nv, cv, dil)."""
+    row = []
+    for lay in layers:
+        row += _addresses(lay[:6]) + [int(v) for v in lay[6:]]
+    _check(load().eemd_sg_backward_layers((c_int64 * len(row))(*row), len(layers), B, T, int(tensor_cores), _p(err),
+                                          _stream()), "eemd_sg_backward_layers")
 
 
 def bias(b, out, n_rows, nv, project=False):

@@ -2092,6 +2092,38 @@ int32_t eemd_sg_wgrad(const void* dy, const void* x, float* dw, float* db, int32
     return cudaGetLastError() == cudaSuccess ? EEMD_SG_OK : EEMD_SG_E_CUDA;
 }
 
+int32_t eemd_sg_forward_layers(const int64_t* table, int32_t n_layers, int32_t B, int32_t T, int32_t tensor_cores,
+                               int32_t* err, void* stream) {
+    if (!table || n_layers < 1) return EEMD_SG_E_BADARG;
+    const auto ptr = [](int64_t v) { return reinterpret_cast<void*>(v); };
+    for (int i = 0; i < n_layers; ++i) {
+        const int64_t* t = table + 10 * i;
+        const int rc = eemd_sg_conv(ptr(t[0]), ptr(t[1]), static_cast<const float*>(ptr(t[2])), ptr(t[3]), B, T,
+                                    (int32_t)t[5], (int32_t)t[6], (int32_t)t[7], (int32_t)t[8], (int32_t)t[9],
+                                    ptr(t[4]), tensor_cores, err, 0, stream);
+        if (rc) return rc;
+    }
+    return EEMD_SG_OK;
+}
+
+int32_t eemd_sg_backward_layers(const int64_t* table, int32_t n_layers, int32_t B, int32_t T, int32_t tensor_cores,
+                                int32_t* err, void* stream) {
+    if (!table || n_layers < 1) return EEMD_SG_E_BADARG;
+    const auto ptr = [](int64_t v) { return reinterpret_cast<void*>(v); };
+    for (int i = 0; i < n_layers; ++i) {
+        const int64_t* t = table + 11 * i;
+        const int32_t rows = (int32_t)t[6], c = (int32_t)t[7], dil = (int32_t)t[10];
+        int rc = eemd_sg_wgrad(ptr(t[0]), ptr(t[1]), static_cast<float*>(ptr(t[2])), static_cast<float*>(ptr(t[3])), B,
+                               T, rows, c, (int32_t)t[8], (int32_t)t[9], dil, tensor_cores != 0, nullptr, 0, stream);
+        // the input gradient times the ReLU derivative of the layer below (its output > 0)
+        if (!rc && t[5])
+            rc = eemd_sg_conv(ptr(t[0]), ptr(t[4]), nullptr, ptr(t[5]), B, T, rows, c, dil, -1, 0, ptr(t[1]),
+                              tensor_cores, err, 0, stream);
+        if (rc) return rc;
+    }
+    return EEMD_SG_OK;
+}
+
 int32_t eemd_sg_loss(const void* out, const void* base, const void* target, void* dout, float* loss, int32_t B,
                      int32_t T, int32_t c, int32_t cv, int32_t margin, int32_t project, float delta,
                      const float* channel_weight, void* stream) {

@@ -172,7 +172,7 @@ class Net:
         self.work = torch.zeros((1,), dtype=torch.float32, device="cuda")
         self.io_increase = None  # calibrated gate bound (load_model / fit)
         # eemd_sg_conv's tensor_cores: 4 warp-specialised with swizzled operands (the fastest:
-        # the 8-layer pass over 16 x 65536 samples in 0.54 ms with it on the 64-channel
+        # the 8-layer pass over 16 x 65536 samples in 0.46 ms with it on the 64-channel
         # inputs, against 1.29 ms for 3, double-buffered with bulk-tensor loads, and 1.47 (2)
         # and 1.71 (1)); all four bit-identical
         self.conv_kernel = 4
@@ -183,47 +183,41 @@ class Net:
         SG.pack_layers([(lay["w"], lay["b"], lay["wp"], lay["wt"], lay["bias"], lay["cout_p"], lay["cin_p"],
                          lay["cout_v"], lay["cin_v"], lay["project"]) for lay in self.layers])
 
-    def layer(self, i, src, dst, B, T, tensor_cores=True):
-        lay = self.layers[i]
-        mode = self.conv_kernel if tensor_cores else 0
-        SG.conv(src, lay["wp"], lay["bias"], dst, B, T, lay["cin_p"], lay["cout_p"], lay["dil"], relu=lay["relu"],
-                tensor_cores=mode, err=self.err)
+    def layers_on(self, bufs, B, T, tensor_cores=True):
+        """Layer i from bufs[i] to bufs[i + 1], all launched by one call (a call
+        and its arguments from Python per layer took longer than a layer of a
+        training step runs)."""
+        SG.forward_layers([(bufs[i], lay["wp"], lay["bias"], bufs[i + 1], None, lay["cin_p"], lay["cout_p"],
+                            lay["dil"], 1, lay["relu"]) for i, lay in enumerate(self.layers)], B, T,
+                          tensor_cores=self.conv_kernel if tensor_cores else 0, err=self.err)
 
     def forward(self, x, B, T, tensor_cores=True):
         """x: bf16 [B][T][CH] -> the activations (x, a1, ..., a8), kept for backward."""
         acts = [x]
-        for i, lay in enumerate(self.layers):
-            y = self.torch.empty((B, T, lay["cout_p"]), dtype=self.torch.bfloat16, device="cuda")
-            self.layer(i, acts[-1], y, B, T, tensor_cores)
-            acts.append(y)
+        for lay in self.layers:
+            acts.append(self.torch.empty((B, T, lay["cout_p"]), dtype=self.torch.bfloat16, device="cuda"))
+        self.layers_on(acts, B, T, tensor_cores)
         return acts
 
     def infer(self, x, out, S, T, chunk, bufs):
         """out[S][T][CH] = net(x[S][T][CH]) over chunks of `chunk` signals with
         two activation buffers bufs[0..1] of [chunk][T][HIDDEN] (nothing kept)."""
-        last = len(self.layers) - 1
+        n = len(self.layers)
         for c0 in range(0, S, chunk):
             cs = min(chunk, S - c0)
-            src = x[c0:c0 + cs]
-            for i in range(len(self.layers)):
-                dst = out[c0:c0 + cs] if i == last else bufs[i & 1][:cs]
-                self.layer(i, src, dst, cs, T)
-                src = dst
+            self.layers_on([x[c0:c0 + cs]] + [bufs[i & 1][:cs] for i in range(n - 1)] + [out[c0:c0 + cs]], cs, T)
 
     def backward(self, acts, dout, B, T, tensor_cores=True):
         """Gradients of every layer from dL/d(output) (the loss kernel's dout)."""
         self.grads.zero_()
-        g = dout
+        g, rows = dout, []
         for li in range(len(self.layers) - 1, -1, -1):
             lay = self.layers[li]
-            SG.wgrad(g, acts[li], lay["dw"], lay["db"], B, T, lay["cout_p"], lay["cin_p"], lay["cout_v"],
-                     lay["cin_v"], lay["dil"], tensor_cores=tensor_cores)
-            if li > 0:
-                gi = self.torch.empty((B, T, lay["cin_p"]), dtype=self.torch.bfloat16, device="cuda")
-                # the input gradient times the ReLU derivative of the layer below (its output > 0)
-                SG.conv(g, lay["wt"], None, gi, B, T, lay["cout_p"], lay["cin_p"], lay["dil"], direction=-1,
-                        mask=acts[li], tensor_cores=self.conv_kernel if tensor_cores else 0, err=self.err)
-                g = gi
+            gi = self.torch.empty((B, T, lay["cin_p"]), dtype=self.torch.bfloat16, device="cuda") if li > 0 else None
+            rows.append((g, acts[li], lay["dw"], lay["db"], lay["wt"], gi, lay["cout_p"], lay["cin_p"], lay["cout_v"],
+                         lay["cin_v"], lay["dil"]))
+            g = gi
+        SG.backward_layers(rows, B, T, tensor_cores=self.conv_kernel if tensor_cores else 0, err=self.err)
 
     def adam_step(self, lr, max_norm=CLIP):
         self.step_count += 1

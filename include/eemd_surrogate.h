@@ -68,6 +68,21 @@ int32_t eemd_sg_bias(const float* b, float* bias, int32_t n_rows, int32_t nv, in
  * and the padded bias, then n_rows, c, nv, cv and project. */
 int32_t eemd_sg_pack_layers(const int64_t* table, int32_t n_layers, void* stream);
 
+/* The kernels of a network's pass, launched by one call.  table (host, read
+ * during the call) gives per layer, in the order of the launches,
+ *   forward  (10 values): eemd_sg_conv's in, w_packed, bias, out, mask (device
+ *            addresses, 0 for none), cin, cout, dil, dir, relu;
+ *   backward (11 values): dy, x, dw, db, the input-gradient operand, dx (device
+ *            addresses; dx = 0: no input gradient), n_rows, c, nv, cv, dil:
+ *            eemd_sg_wgrad, then eemd_sg_conv of dy (dir -1, mask x) into dx.
+ * tensor_cores as eemd_sg_conv takes it (in the backward pass the weight
+ * gradient runs on the tensor cores when it is not 0).  A refused layer ends
+ * the call with its status; the layers before it have been launched. */
+int32_t eemd_sg_forward_layers(const int64_t* table, int32_t n_layers, int32_t B, int32_t T, int32_t tensor_cores,
+                               int32_t* err, void* stream);
+int32_t eemd_sg_backward_layers(const int64_t* table, int32_t n_layers, int32_t B, int32_t T, int32_t tensor_cores,
+                                int32_t* err, void* stream);
+
 /* Accumulates dw[n][tap][c] += sum_t dy[b][t][n] * x[b][t+(tap-1)*dil][c]
  * (n < nv, c < cv) and db[n] += sum_t dy[b][t][n]; dy is [B][T][n_rows],
  * x is [B][T][c] (both bf16, n_rows, c <= 64).  tensor_cores != 0 (and n_rows

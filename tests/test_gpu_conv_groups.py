@@ -62,3 +62,46 @@ def test_loss_turns(B, T, project, delta):
         grad[..., :cv] -= grad.sum(-1, keepdims=True) / cv
     assert abs(float(acc.item()) - loss) <= 1e-5 * loss
     assert np.max(np.abs(dout.double().cpu().numpy() - grad)) <= 2 ** -8 * np.max(np.abs(grad))
+
+
+@pytest.mark.parametrize("tensor_cores", [True, False])
+def test_passes_in_one_call_equal_layer_by_layer(tensor_cores):
+    """A network's forward and backward pass against the same kernels called
+    one by one: the same activations, and gradients within the float32 rounding
+    of sums added in another order (B T products, as the weight-gradient tests)."""
+    from eemd4cuda_b200 import surrogate as SU
+
+    B, T = 2, 300
+    net = SU.Net(seed=3)
+    g = torch.Generator().manual_seed(1)
+    x = torch.randn((B, T, SU.CH), generator=g).to(torch.bfloat16).cuda()
+    dout = torch.randn((B, T, SU.CH), generator=g).to(torch.bfloat16).cuda()
+    acts = net.forward(x, B, T, tensor_cores)
+    net.backward(acts, dout, B, T, tensor_cores)
+    mode = net.conv_kernel if tensor_cores else 0
+    got, src, dy = net.grads.clone(), x, dout
+    for i, lay in enumerate(net.layers):
+        y = torch.empty_like(acts[i + 1])
+        _sg.conv(src, lay["wp"], lay["bias"], y, B, T, lay["cin_p"], lay["cout_p"], lay["dil"], relu=lay["relu"],
+                 tensor_cores=mode, err=net.err)
+        assert torch.equal(y, acts[i + 1])
+        src = y
+    net.grads.zero_()
+    for i in range(len(net.layers) - 1, -1, -1):
+        lay = net.layers[i]
+        _sg.wgrad(dy, acts[i], lay["dw"], lay["db"], B, T, lay["cout_p"], lay["cin_p"], lay["cout_v"], lay["cin_v"],
+                  lay["dil"], tensor_cores=tensor_cores)
+        dx = torch.empty((B, T, lay["cin_p"]), dtype=torch.bfloat16, device="cuda")
+        _sg.conv(dy, lay["wt"], None, dx, B, T, lay["cout_p"], lay["cin_p"], lay["dil"], direction=-1, mask=acts[i],
+                 tensor_cores=mode, err=net.err)
+        dy = dx
+    net.check()
+    scale = float(net.grads.abs().max())
+    assert scale > 0 and float((got - net.grads).abs().max()) <= 4e-5 * np.sqrt(B * T) * scale
+
+
+def test_a_refused_layer_ends_the_pass():
+    x = torch.zeros((1, 64, 16), dtype=torch.bfloat16, device="cuda")
+    with pytest.raises(_sg.SurrogateError) as e:
+        _sg.forward_layers([(x, x, None, x, None, 16, 48, 1, 1, False)], 1, 64, tensor_cores=4)
+    assert e.value.status == _sg.SG_E_BADARG
