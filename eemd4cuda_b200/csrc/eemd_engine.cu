@@ -14,8 +14,9 @@
 // (separately rounded products, IEEE divisions, serial-Thomas recurrences;
 // the file is compiled with --fmad=false so the compiler never contracts
 // a*b+c).  exact=0 uses explicit fma(), a Newton-refined reciprocal per row,
-// a twisted (two-sided) seam-window factorisation held in registers, and the
-// monomial form of each spline interval.
+// a seam-window elimination of five rows per lane whose forward (c, d) meet
+// the neighbouring lanes' in shared memory, and the monomial form of each
+// spline interval.
 #include "../../include/eemd_b200.h"
 #include "eemd_internal.cuh"
 

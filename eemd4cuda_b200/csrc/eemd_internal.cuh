@@ -10,7 +10,8 @@
 //
 //   solve   both envelope systems, decay-seamed block Thomas: the windows of
 //           each envelope are split over the cluster's CTAs; knots are staged
-//           in shared memory; second derivatives go to global memory
+//           in shared memory; interval records (exact mode: second
+//           derivatives) go to global memory
 //           (emd_ref.py:31-65, emd_gpu_v5_dsbt.py:51-74)
 //   barrier.cluster (release/acquire)
 //   sweep   each CTA streams its segment tile by tile: spline evaluation of
@@ -23,7 +24,7 @@
 //           memory; barrier.cluster; every CTA reads all C entries through
 //           distributed shared memory and takes the same stop decision
 //
-// Knot lists, second derivatives and solve scratch live in per-cluster-slot
+// Knot lists, interval records and solve scratch live in per-cluster-slot
 // regions of the workspace; residuals and IMFs live per task.
 #pragma once
 #include <stdint.h>

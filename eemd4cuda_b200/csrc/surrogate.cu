@@ -1674,20 +1674,28 @@ __global__ void __launch_bounds__(128) k_combine(const double* __restrict__ imf_
     for (int t = lo + (int)threadIdx.x; t < hi; t += 128) {
         const size_t it = (size_t)s * N + t;
         const __nv_bfloat16* o = net + it * C;
+        // a sample's loads before its first store, which they would otherwise wait
+        // behind one by one (16 x 65536 samples 195 us so, 90 now)
+        double sum[K];
+        float dn[PMAX];
+#pragma unroll
+        for (int m = 0; m < K; ++m) sum[m] = imf_sum[((size_t)s * K + m) * N + t];
+#pragma unroll
+        for (int m = 0; m < PMAX; ++m) dn[m] = m < P ? __bfloat162float(o[m]) : 0.f;
+        const double xv = (double)x[it];
         double c[K + 1], mr[PMAX];
         double acc = 0.0, moved = 0.0, sum_c = 0.0;
 #pragma unroll
         for (int m = 0; m < K; ++m) {
-            const double mean = imf_sum[((size_t)s * K + m) * N + t] / cnt_d[m];
+            const double mean = sum[m] / cnt_d[m];
             if (m < PMAX) mr[m] = mean;
             acc += mean;
-            const double d = m < P ? sc * (double)__bfloat162float(o[m]) : 0.0;
+            const double d = m < P ? sc * (double)dn[m < PMAX ? m : 0] : 0.0;
             moved += d;
             c[m] = mean + d;
             imfs_out[((size_t)s * K + m) * N + t] = c[m];
             sum_c += c[m];
         }
-        const double xv = (double)x[it];
         c[K] = (xv - acc) - moved;
         resid_out[it] = c[K];
         const double e = xv - (sum_c + c[K]);
@@ -1724,15 +1732,23 @@ __global__ void __launch_bounds__(128) k_combine(const double* __restrict__ imf_
 // less that of the small-ensemble modes (or any of these is not finite).
 // Orthogonality index (Huang et al. 1998): sum over pairs j != k of
 // <c_j, c_k> over ||x||^2.
-__global__ void k_gate(const double* __restrict__ partial, int S, int chunks, int P, double recon_bound,
-                       double io_bound, int io_relative, double* metrics, int* fallback) {
+// One CTA per signal, a thread per sum (a thread per signal, all sums one after
+// the other, was 131 us at any batch; 8 so).
+__global__ void __launch_bounds__(128) k_gate(const double* __restrict__ partial, int chunks, int P, double recon_bound,
+                                              double io_bound, int io_relative, double* metrics, int* fallback) {
     constexpr int K = GK;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    double tot[NSTAT];
-    for (int j = 0; j < NSTAT; ++j) tot[j] = 0.0;
-    for (int ch = 0; ch < chunks; ++ch)
-        for (int j = 0; j < NSTAT; ++j) tot[j] += partial[((size_t)s * chunks + ch) * NSTAT + j];
+    static_assert(NSTAT <= 128, "a thread per sum");
+    const int s = blockIdx.x;
+    __shared__ double tot[NSTAT];
+    if (threadIdx.x < NSTAT) {
+        const double* p = partial + (size_t)s * chunks * NSTAT + threadIdx.x;
+        double a = 0.0;
+#pragma unroll 8
+        for (int ch = 0; ch < chunks; ++ch) a += p[(size_t)ch * NSTAT];
+        tot[threadIdx.x] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
     double cross = 0.0, cross_p = 0.0, cross_ref = 0.0;
     int q = 2;
     for (int a = 0; a <= K; ++a)
@@ -2188,8 +2204,7 @@ int32_t eemd_sg_combine(const double* imf_sum, const int32_t* mode_count, const 
     k_combine<<<dim3(chunks, S), 128, 0, st>>>(imf_sum, mode_count, x, scale,
                                                 static_cast<const __nv_bfloat16*>(net_out), imfs_out, resid_out,
                                                 partial, N, C, P);
-    k_gate<<<(S + 127) / 128, 128, 0, st>>>(partial, S, chunks, P, recon_bound, io_bound, io_relative, metrics,
-                                            fallback);
+    k_gate<<<S, 128, 0, st>>>(partial, chunks, P, recon_bound, io_bound, io_relative, metrics, fallback);
     return cudaGetLastError() == cudaSuccess ? EEMD_SG_OK : EEMD_SG_E_CUDA;
 }
 

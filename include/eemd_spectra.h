@@ -11,7 +11,10 @@
  *   eemd_sp_stft        replaces spectra.py:18-29 stft_block:
  *       scipy.signal.stft(window='hann', boundary='zeros', padded=False),
  *       one-sided, divided by the window's sum.
- *   eemd_sp_fft         the complex FFT both use (numpy.fft.fft's convention
+ *       Rows are transformed as real ones (of their own length, or as a circular
+ *       convolution with the closed-form Hilbert kernel where the length has a
+ *       large prime factor), so neither z nor its spectrum is formed.
+ *   eemd_sp_fft         a complex FFT of any length (numpy.fft.fft's convention
  *       for sign -1, unnormalised), this library's own: Stockham passes of
  *       radix 4, 2, 3, 5 and odd primes up to 31, Bluestein's chirp-z for a
  *       length with a larger prime factor.
