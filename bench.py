@@ -379,12 +379,12 @@ def measured_peak_hbm():
 # of the same signal and are scaled per (signal, trial) task, since every task
 # streams its own buffers.
 EMD_TRAFFIC = {
-    "harmonic48k": {"bytes_per_launch": 6837855000,
-                    "engine_sha256": "3788a361741c024d3ab67bed60b11685f8a5f528f948919fb8eb3f3ad6b353ab",
+    "harmonic48k": {"bytes_per_launch": 3122266880,
+                    "engine_sha256": "aef4ddc7a17c12bdf012ed251f5fbcd1deabf298ae186f76a95fcb0171e06e9a",
                     "capture": "one k_emd launch of the 100-trial 48 kHz workload (clusters of 4 five-warp CTAs)"},
-    "amfm4m": {"bytes_per_task": 5603181376.0,
-               "engine_sha256": "3788a361741c024d3ab67bed60b11685f8a5f528f948919fb8eb3f3ad6b353ab",
-               "capture": "one k_emd launch of 4 trials of the 2^22-sample signal (clusters of 16 four-warp "
+    "amfm4m": {"bytes_per_task": 4268230784.0,
+               "engine_sha256": "aef4ddc7a17c12bdf012ed251f5fbcd1deabf298ae186f76a95fcb0171e06e9a",
+               "capture": "one k_emd launch of 4 trials of the 2^22-sample signal (clusters of 16 five-warp "
                           "CTAs), per task"},
 }
 
@@ -1312,14 +1312,26 @@ def fft_passes(n: int) -> int:
 
 
 def spectra_launches(n: int, nperseg: int) -> int:
-    """Launches of the spectra step: two STFT calls (one launch each when the
-    frames are direct lengths up to 4096, else k_frames, the frame FFT and
-    k_stft_out) and one Hilbert call (two four-step transforms with the real
-    input and the analytic weights in their loads, then k_if_amp; else
-    k_promote, FFT, k_analytic, inverse FFT, k_if_amp)."""
+    """Launches of the spectra step through complex transforms of the rows: two
+    STFT calls (one launch each when the frames are direct lengths up to 4096,
+    else k_frames, the frame FFT and k_stft_out) and one Hilbert call (two
+    four-step transforms, then k_if_amp; else k_promote, FFT, k_analytic,
+    inverse FFT, k_if_amp)."""
     stft = 1 if nperseg <= SMEM_FFT_MAX and _fft_radices(nperseg)[1] else 2 + fft_passes(nperseg)
     hilbert = 5 if _fft_radices(n)[1] and fft4_split(n) else 3 + 2 * fft_passes(n)
     return 2 * stft + hilbert
+
+
+def spectra_real_launches(n: int, nperseg: int) -> int:
+    """Launches of the spectra step through real transforms, the path of frames
+    of up to 4096 samples and rows of up to 8 million: one per STFT call, and
+    per Hilbert call columns, rows, columns and the closing kernel (one launch
+    for rows of up to 2048 complex points), after the transform of the
+    convolution kernel where the row's half length is not a direct one."""
+    stft = 2 if nperseg <= SMEM_FFT_MAX and _fft_radices(nperseg)[1] else 2 * (2 + fft_passes(nperseg))
+    if n % 2 == 0 and _fft_radices(n // 2)[1]:
+        return stft + (1 if n // 2 <= 2048 else 4)
+    return stft + (2 if n <= 2048 else 6)
 
 
 def run_spectra(args):
@@ -1418,9 +1430,9 @@ def run_spectra(args):
         "e2e": {"value": round(rows * N / (e2e / 1e3) / 1e6, 3), "unit": "Msamples/s", "ms_per_step": round(e2e, 3),
                 "h2d_bytes_per_step": rows * N * 8 + r.n_modes * N * 8,
                 "d2h_bytes_per_step": rows * F * T * 16 + 2 * r.n_modes * N * 8},
-        "gpu_launches": spectra_launches(N, nper) * args.steps,
-        "roofline": {"bound": "hbm", "kernel": "hilbert stage (four-step FFT with the real input in its loads, "
-                                               "inverse four-step FFT with the analytic weights, k_if_amp)",
+        "gpu_launches": spectra_real_launches(N, nper) * args.steps,
+        "roofline": {"bound": "hbm", "kernel": "hilbert stage (k_hil_cols, k_hil_rows, k_hil_cols, k_hil_out: the "
+                                               "Hilbert transform through real transforms of half length)",
                      "achieved": round(gbs, 2), "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": round(gbs / peak, 4), "traffic": None, "algorithmic_bytes": h_bytes,
                      "ms": round(h_ms, 4)},
