@@ -1265,8 +1265,12 @@ __global__ void __launch_bounds__(NT) k_wgrad_tc(const __nv_bfloat16* __restrict
 //   4 warps   : add the tile's dy rows up for the bias gradient (in float32, on
 //               CUDA cores) and release the stage; after the last tile read the
 //               accumulators and add them to dw
-// Bound by the L2 traffic of four boxes per tile.  32 x 4096 samples, 64 to 64
-// channels: 100 us with k_wgrad_tc, 19.5 us here.  Every wait is bounded.
+// Bound by shared memory (per tile 96 KB of operand reads, 64 KB of copies, 16 KB
+// for the bias sums: 0.7 us) and by the first copies of a CTA that has 7 tiles.
+// 32 x 4096 samples, 64 to 64 channels: 100 us with k_wgrad_tc, 19.5 us here.
+// Over a step of 363 us: a quarter of the MMAs, or an eighth of the sums' reads,
+// 345; one box for the three taps (2.7 times fewer bytes from L2) 365; twice the
+// summing warps 363; no atomics on dw 360.  Every wait is bounded.
 constexpr int WG_SUM = 4;                       // summing warps
 constexpr int WG_THREADS = 32 * (WG_SUM + 2);
 
