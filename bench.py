@@ -1326,12 +1326,12 @@ def spectra_real_launches(n: int, nperseg: int) -> int:
     """Launches of the spectra step through real transforms, the path of frames
     of up to 4096 samples and rows of up to 8 million: one per STFT call, and
     per Hilbert call columns, rows, columns and the closing kernel (one launch
-    for rows of up to 2048 complex points), after the transform of the
-    convolution kernel where the row's half length is not a direct one."""
+    for rows of up to 2048 complex points), and one more for the transform of
+    the convolution kernel where the row's half length is not a direct one."""
     stft = 2 if nperseg <= SMEM_FFT_MAX and _fft_radices(nperseg)[1] else 2 * (2 + fft_passes(nperseg))
     if n % 2 == 0 and _fft_radices(n // 2)[1]:
         return stft + (1 if n // 2 <= 2048 else 4)
-    return stft + (2 if n <= 2048 else 6)
+    return stft + (2 if n <= 2048 else 5)
 
 
 def run_spectra(args):

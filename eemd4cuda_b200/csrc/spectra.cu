@@ -606,8 +606,8 @@ __global__ void __launch_bounds__(FFT_THREADS, 1) k_fft4_rows(const double2* __r
 // lie in rows k1 and N1 - k1, which one CTA holds), columns back.  Rows of
 // h <= HIL_SMALL points take one launch.
 // Against complex transforms of the rows, Bluestein's for a length with a large
-// prime factor (B200): 10 rows of 441 003 samples 3790 -> 441 us, 10 of 441 000
-// 1367 -> 407 us, 8 of 48 000 78 -> 42 us, 16 of 4963 224 -> 49 us.
+// prime factor (B200): 10 rows of 441 003 samples 3790 -> 421 us, 10 of 441 000
+// 1367 -> 407 us, 8 of 48 000 78 -> 42 us, 16 of 4963 224 -> 47 us.
 // ---------------------------------------------------------------------------
 constexpr int HIL_SMALL = 2048;
 
@@ -674,11 +674,13 @@ __device__ __forceinline__ double2 hil_imag(double2 a, double2 b, double2 w) {
     return make_double2(E.y + wO.y, -(E.y - wO.y));
 }
 
-// columns: forward from the samples (x, or the kernel when x is null) into
-// Y[m][k1][n2], or (INV) back from Y into the samples of out
+// columns: forward from the samples into Y[m][k1][n2] and, where g takes a
+// transform, from the kernel into Yk first, or (INV) back from Y into the samples
+// of out.  A launch of its own for the kernel was one more latency: 10 rows of
+// 441 003 samples 437 -> 421 us, 2 of 100 003 66 -> 57, 9 of 7159 52 -> 46.
 template <bool INV, int P>
-__global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_cols(const double* __restrict__ x, double2* Y, double* out, int M,
-                                                          const __grid_constant__ HilPlan F) {
+__global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_cols(const double* __restrict__ x, double2* Y, double2* Yk,
+                                                          double* out, int M, const __grid_constant__ HilPlan F) {
     extern __shared__ double2 sfft[];
     const int N1 = F.p1.n, N2 = F.p2.n, CB = F.cb, ld = pad8(N1 + 8), lg = __ffs(CB) - 1;
     double2* a = sfft;
@@ -686,11 +688,13 @@ __global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_cols(const double* __res
     double2* tw = tab + ld;
     make_table<false>(tab, N1);
     after_previous_kernel();
-    const int nblk = (N2 + CB - 1) / CB;
-    for (int64_t blk = blockIdx.x; blk < (int64_t)M * nblk; blk += gridDim.x) {
-        const int64_t m = blk / nblk;
+    const int nblk = (N2 + CB - 1) / CB, first = !INV && F.conv ? 1 : 0;  // (row 0 is the kernel)
+    for (int64_t blk = blockIdx.x; blk < (int64_t)(M + first) * nblk; blk += gridDim.x) {
+        const int64_t m = blk / nblk - first;
         const int c0 = (int)(blk % nblk) * CB;
         const int cb = min(CB, N2 - c0);
+        const double* xr = INV || m < 0 ? nullptr : x + m * F.N;
+        double2* Yr = m < 0 ? Yk : Y + m * F.h;
         make_col_twiddles(tw, N1, cb, c0, F.h);
         if (INV) __syncthreads();
         for (int i = threadIdx.x; i < N1 << lg; i += blockDim.x) {
@@ -698,8 +702,8 @@ __global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_cols(const double* __res
             double2 v = make_double2(0.0, 0.0);
             if (c < cb) {
                 const int64_t n = (int64_t)n1 * N2 + c0 + c;
-                if (INV) v = cmul(Y[m * F.h + n], col_twiddle(tw, N1, c, n1, +1));  // (n1 is k1 here)
-                else v = hil_point(x ? x + m * F.N : nullptr, F.N, 2 * F.h, n);
+                if (INV) v = cmul(Yr[n], col_twiddle(tw, N1, c, n1, +1));  // (n1 is k1 here)
+                else v = hil_point(xr, F.N, 2 * F.h, n);
             }
             a[c * ld + pad8(n1)] = v;
         }
@@ -715,7 +719,7 @@ __global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_cols(const double* __res
                 if (2 * n < F.N) o[0] = v.x;
                 if (2 * n + 1 < F.N) o[1] = v.y;
             } else {
-                Y[m * F.h + n] = cmul(v, col_twiddle(tw, N1, c, k1, -1));
+                Yr[n] = cmul(v, col_twiddle(tw, N1, c, k1, -1));
             }
         }
         __syncthreads();
@@ -1295,14 +1299,11 @@ int hil_launch(const double* x, int M, double sr, double* freq, double* amp, voi
     const size_t sr_ = (size_t)(2 * F.ub + 1) * pad8(F.p2.n + 8) * sizeof(double2) + F.ub * sizeof(double2);
     const int tc = fft_threads(F.p1, F.cb, P), tr = fft_threads(F.p2, 2 * F.ub, P);
     const int64_t bc = (F.p2.n + F.cb - 1) / F.cb, br = (F.p1.n / 2 + 1 + F.ub - 1) / F.ub;
-    if (F.conv) {
-        double2* Yk = reinterpret_cast<double2*>(base);
-        launch_after(k_hil_cols<false, P>, smem_grid(bc), tc, sc, st, static_cast<double*>(nullptr), Yk, static_cast<double*>(nullptr), 1, F);
-        launch_after(k_hil_rows<true, P>, smem_grid(br), tr, sr_, st, Yk, g, 1, F);
-    }
-    launch_after(k_hil_cols<false, P>, smem_grid(bc * M), tc, sc, st, x, Y, static_cast<double*>(nullptr), M, F);
+    double2* Yk = reinterpret_cast<double2*>(base);  // (conv)
+    launch_after(k_hil_cols<false, P>, smem_grid(bc * (M + (F.conv ? 1 : 0))), tc, sc, st, x, Y, Yk, static_cast<double*>(nullptr), M, F);
+    if (F.conv) launch_after(k_hil_rows<true, P>, smem_grid(br), tr, sr_, st, Yk, g, 1, F);
     launch_after(k_hil_rows<false, P>, smem_grid(br * M), tr, sr_, st, Y, g, M, F);
-    launch_after(k_hil_cols<true, P>, smem_grid(bc * M), tc, sc, st, static_cast<double*>(nullptr), Y, hx, M, F);
+    launch_after(k_hil_cols<true, P>, smem_grid(bc * M), tc, sc, st, static_cast<double*>(nullptr), Y, static_cast<double2*>(nullptr), hx, M, F);
     launch_after(k_hil_out, smem_grid(((F.N + IF_TILE - 1) / IF_TILE) * M), IF_THREADS, 0, st, x, hx, freq, amp, M, F.N, sr);
     return EEMD_SP_OK;
 }
