@@ -1246,6 +1246,12 @@ bool hil_plan(int64_t N, HilPlan& F) {
 
 bool hil_small(const HilPlan& F) { return F.p1.n == 1; }
 
+// whether [a, a + na) and [b, b + nb) share a byte
+bool overlaps(const void* a, size_t na, const void* b, size_t nb) {
+    const uintptr_t pa = reinterpret_cast<uintptr_t>(a), pb = reinterpret_cast<uintptr_t>(b);
+    return pa < pb + nb && pb < pa + na;
+}
+
 // workspace of the plan: Y, the kernel's Y and g, the rows' Hilbert transforms
 size_t hil_bytes(const HilPlan& F, int64_t M) {
     const size_t gb = F.conv ? al((size_t)(F.h + 1) * sizeof(double)) : 0;
@@ -1487,8 +1493,18 @@ int32_t eemd_sp_hilbert_if(const double* x, int32_t M, int64_t N, double sr, dou
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const Bufs b = carve(ws, L);
     const int64_t total = (int64_t)M * N;
+    // the real transforms' last kernel reads the rows (and a tile's neighbours) while it
+    // writes the outputs: rows that share memory with an output are copied first
+    const size_t nb = sizeof(double) * (size_t)total;
+    const bool in_place = overlaps(x, nb, inst_freq, nb) || overlaps(x, nb, inst_amp, nb);
+    const size_t copy = in_place ? al(nb) : 0;
     HilPlan F;
-    if (hil_plan(N, F) && hil_bytes(F, M) <= ws_bytes) {
+    if (hil_plan(N, F) && copy + hil_bytes(F, M) <= ws_bytes) {
+        if (in_place) {
+            if (cudaMemcpyAsync(ws, x, nb, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return EEMD_SP_E_CUDA;
+            x = static_cast<const double*>(ws);
+            ws = static_cast<char*>(ws) + copy;
+        }
         const int r = hil_run(x, M, sr, inst_freq, inst_amp, ws, F, st);
         if (r) return r;
         return cudaGetLastError() == cudaSuccess ? EEMD_SP_OK : EEMD_SP_E_CUDA;

@@ -55,7 +55,8 @@ int32_t eemd_sp_fft(const double* in, double* out, int32_t M, int64_t N, int32_t
 /* Workspace bytes for eemd_sp_hilbert_if on M rows of N samples. */
 int32_t eemd_sp_hilbert_workspace(int32_t M, int64_t N, size_t* bytes);
 
-/* inst_freq[m][n] (Hz) and inst_amp[m][n] of every row x[m][:] (N >= 2). */
+/* inst_freq[m][n] (Hz) and inst_amp[m][n] of every row x[m][:] (N >= 2).
+ * Either output may be x or overlap it; the two outputs and the workspace are apart. */
 int32_t eemd_sp_hilbert_if(const double* x, int32_t M, int64_t N, double sr, double* inst_freq, double* inst_amp,
                            void* ws, size_t ws_bytes, void* stream);
 
