@@ -814,6 +814,11 @@ __device__ __forceinline__ double gradient(double pl, double p, double pr, bool 
     return f * (0.5 / PI);
 }
 
+// arg(z) of a sample.  A zero sample counts as +0 whatever its sign, as a sum
+// over a transform's terms gives it: where the row and its transform are zero
+// the phase is then zero too (a negative zero would make it +-pi).
+__device__ __forceinline__ double phase_of(double re, double im) { return atan2(im, re + 0.0); }
+
 // |z| of a sample: the root of the squares' sum where they neither overflow nor
 // underflow, hypot elsewhere; a row with a non-finite sample has no finite
 // transform, so its magnitude is not a number throughout, as with a transform
@@ -839,9 +844,9 @@ __global__ void __launch_bounds__(IF_THREADS) k_hil_out(const double* __restrict
         const int n = (int)min((int64_t)IF_TILE, N - t0);
         const double* xr = x + m * N + t0;
         const double* hr = hx + m * N + t0;
-        for (int i = threadIdx.x; i < n; i += IF_THREADS) ph[i + 1] = atan2(hr[i], xr[i]);
-        if (threadIdx.x == IF_THREADS - 1 && t0 > 0) ph[0] = atan2(hr[-1], xr[-1]);
-        if (threadIdx.x == IF_THREADS - 33 && t0 + n < N) ph[n + 1] = atan2(hr[n], xr[n]);
+        for (int i = threadIdx.x; i < n; i += IF_THREADS) ph[i + 1] = phase_of(xr[i], hr[i]);
+        if (threadIdx.x == IF_THREADS - 1 && t0 > 0) ph[0] = phase_of(xr[-1], hr[-1]);
+        if (threadIdx.x == IF_THREADS - 33 && t0 + n < N) ph[n + 1] = phase_of(xr[n], hr[n]);
         __syncthreads();
         for (int i = threadIdx.x; i < n; i += IF_THREADS) {
             const int64_t t = t0 + i;
@@ -894,7 +899,7 @@ __global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_small(const double* __re
         if (!SPEC) {
             smem_fft<true, P>(a, half, F.p2, +1, 1, 0);
             auto im_at = [&](int t) { return (t & 1) ? a[pad8(t >> 1)].y : a[pad8(t >> 1)].x; };
-            for (int t = threadIdx.x; t < N; t += blockDim.x) ph[t] = atan2(im_at(t), xr[t]);
+            for (int t = threadIdx.x; t < N; t += blockDim.x) ph[t] = phase_of(xr[t], im_at(t));
             __syncthreads();
             for (int t = threadIdx.x; t < N; t += blockDim.x) {
                 inst_freq[(int64_t)m * N + t] = gradient(t > 0 ? ph[t - 1] : 0.0, ph[t], t + 1 < N ? ph[t + 1] : 0.0,
