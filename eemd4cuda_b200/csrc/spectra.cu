@@ -887,7 +887,9 @@ __global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_small(const double* __re
                     g[h - k] = gi.y * inv;
                 }
             } else if (k == 0) {
-                *za = make_double2(0.0, 0.0);
+                // (zero, and not a number where a sample is not finite: the only bin of two samples)
+                const double z = (za->x - za->x) + (za->y - za->y);
+                *za = make_double2(z, z);
             } else {
                 double2 va = *za, vb = *zb;
                 hil_pair(va, vb, F.conv ? g[k] : -inv, F.conv ? g[h - k] : -inv, w);

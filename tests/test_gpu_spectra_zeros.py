@@ -22,3 +22,15 @@ def test_zero_rows_of_either_sign(N):
     X[3, 1::2] = -0.0
     f, a = hilbert(X)
     assert not f.any() and not a.any()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("N", [2, 3, 4, 5, 4098])
+def test_rows_with_a_non_finite_sample(N, bad):
+    """Such a row has no finite transform; the row beside it keeps its own."""
+    X = np.random.default_rng(N).standard_normal((3, N))
+    f0, a0 = hilbert(X)
+    X[0, 0] = X[1, N - 1] = bad
+    f, a = hilbert(X)
+    assert not np.isfinite(f[:2]).any() and not np.isfinite(a[:2]).any()
+    assert np.array_equal(f[2], f0[2]) and np.array_equal(a[2], a0[2])
