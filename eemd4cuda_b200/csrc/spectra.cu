@@ -333,6 +333,8 @@ struct SmemPlan {
 // launches: each makes its tables while the one before drains, then waits for
 // it here before the first access to what it wrote (or to what its own writes
 // would overwrite).
+// (A kernel's life then overlaps that kernel's writes: no const __restrict__
+// pointers and no __ldg here, whose loads presume memory that stays unchanged.)
 __device__ __forceinline__ void after_previous_kernel() {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -679,7 +681,7 @@ __device__ __forceinline__ double2 hil_imag(double2 a, double2 b, double2 w) {
 // of out.  A launch of its own for the kernel was one more latency: 10 rows of
 // 441 003 samples 437 -> 421 us, 2 of 100 003 66 -> 57, 9 of 7159 52 -> 46.
 template <bool INV, int P>
-__global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_cols(const double* __restrict__ x, double2* Y, double2* Yk,
+__global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_cols(const double* x, double2* Y, double2* Yk,
                                                           double* out, int M, const __grid_constant__ HilPlan F) {
     extern __shared__ double2 sfft[];
     const int N1 = F.p1.n, N2 = F.p2.n, CB = F.cb, ld = pad8(N1 + 8), lg = __ffs(CB) - 1;
@@ -833,7 +835,7 @@ __device__ __forceinline__ double magnitude(double re, double im) {
 // phase is formed once (and twice at a tile's two ends), not by each of the
 // three samples that read it; bound by the arc tangents' instructions
 constexpr int IF_THREADS = 256, IF_TILE = 4 * IF_THREADS;
-__global__ void __launch_bounds__(IF_THREADS) k_hil_out(const double* __restrict__ x, const double* __restrict__ hx,
+__global__ void __launch_bounds__(IF_THREADS) k_hil_out(const double* x, const double* hx,
                                                         double* inst_freq, double* inst_amp, int M, int64_t N,
                                                         double sr) {
     __shared__ double ph[IF_TILE + 2];
@@ -860,7 +862,7 @@ __global__ void __launch_bounds__(IF_THREADS) k_hil_out(const double* __restrict
 // h <= HIL_SMALL: the whole row in one CTA iteration (g: the kernel's transform
 // from a launch with x null and M = 1, or unread when L = N)
 template <bool SPEC, int P>
-__global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_small(const double* __restrict__ x, double* g, double* inst_freq,
+__global__ void __launch_bounds__(FFT_THREADS, 1) k_hil_small(const double* x, double* g, double* inst_freq,
                                                            double* inst_amp, int M, double sr,
                                                            const __grid_constant__ HilPlan F) {
     extern __shared__ double2 sfft[];

@@ -47,6 +47,8 @@ __device__ __forceinline__ void raise(int* err, int code) {
 // kernel drains (programmatic dependent launch: its own start-up then overlaps
 // that kernel's tail); they wait here before their first access to memory that
 // it may have written or still reads.
+// (A kernel's life then overlaps that kernel's writes: no const __restrict__
+// pointers and no __ldg here, whose loads presume memory that stays unchanged.)
 __device__ __forceinline__ void after_previous_kernel() {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -737,10 +739,10 @@ __device__ __forceinline__ bool epi_bar_or(int grp, bool v) {
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant__ CUtensorMap tin,
                                                             const __grid_constant__ CUtensorMap tout,
-                                                            const __nv_bfloat16* __restrict__ wpk,
-                                                            const float* __restrict__ bias, int B, int T, int dil,
+                                                            const __nv_bfloat16* wpk,
+                                                            const float* bias, int B, int T, int dil,
                                                             int dir, int relu,
-                                                            const __nv_bfloat16* __restrict__ mask, int* err,
+                                                            const __nv_bfloat16* mask, int* err,
                                                             long long spin_limit) {
     using G = WsGeo<CIN, COUT>;
     constexpr int NS = WS_STAGES;
@@ -980,7 +982,7 @@ __global__ void k_conv_ref(const __nv_bfloat16* __restrict__ in, const __nv_bflo
 // subtracts from every weight the mean over the output channels of the
 // forward layer (n for transpose = 0, c for transpose = 1): the layer's
 // outputs then sum to zero over those channels.
-__device__ __forceinline__ void pack_element(int i, const float* __restrict__ w, __nv_bfloat16* wpk, int N, int C,
+__device__ __forceinline__ void pack_element(int i, const float* w, __nv_bfloat16* wpk, int N, int C,
                                              int nv, int cv, int transpose, int project) {
     const int n = i / (3 * C), k = i % (3 * C);
     const int tap = k / C, c = k % C;
@@ -1005,7 +1007,7 @@ __global__ void k_pack(const float* __restrict__ w, __nv_bfloat16* wpk, int N, i
 }
 
 // bias[n] = b[n] (n < nv, minus the mean over nv when project), 0 up to N
-__device__ __forceinline__ void bias_element(int n, const float* __restrict__ b, float* bias, int nv, int project) {
+__device__ __forceinline__ void bias_element(int n, const float* b, float* bias, int nv, int project) {
     float s = 0.f;
     if (project)
         for (int q = 0; q < nv; ++q) s += b[q];
@@ -1475,10 +1477,10 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constan
 // project = 1 (C = 16) removes the mean over the cv channels from the
 // gradient of every sample: the gradient with respect to the raw output of a
 // layer whose outputs are projected onto zero channel sum.
-__global__ void k_loss(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ base,
-                       const __nv_bfloat16* __restrict__ target, __nv_bfloat16* dout, float* loss, int B, int T,
+__global__ void k_loss(const __nv_bfloat16* out, const __nv_bfloat16* base,
+                       const __nv_bfloat16* target, __nv_bfloat16* dout, float* loss, int B, int T,
                        int C, int cv, int margin, float inv_count, int project, float delta,
-                       const float* __restrict__ wch) {
+                       const float* wch) {
     __shared__ float part[8];
     after_previous_kernel();
     const long long n = (long long)B * T * C;
@@ -1566,7 +1568,7 @@ __global__ void k_adam(float* p, const float* g, float* m, float* v, int n, floa
 }
 
 // out[0] = sum of g[i]^2 (one CTA, fixed order)
-__global__ void __launch_bounds__(1024) k_sumsq(const float* __restrict__ g, int n, float* out) {
+__global__ void __launch_bounds__(1024) k_sumsq(const float* g, int n, float* out) {
     __shared__ float part[32];
     after_previous_kernel();
     float a = 0.f;
