@@ -2136,7 +2136,7 @@ int32_t eemd_sg_backward_layers(const int64_t* table, int32_t n_layers, int32_t 
         const int64_t* t = table + 11 * i;
         const int32_t rows = (int32_t)t[6], c = (int32_t)t[7], dil = (int32_t)t[10];
         int rc = eemd_sg_wgrad(ptr(t[0]), ptr(t[1]), static_cast<float*>(ptr(t[2])), static_cast<float*>(ptr(t[3])), B,
-                               T, rows, c, (int32_t)t[8], (int32_t)t[9], dil, tensor_cores != 0, nullptr, 0, stream);
+                               T, rows, c, (int32_t)t[8], (int32_t)t[9], dil, tensor_cores != 0, err, 0, stream);
         // the input gradient times the ReLU derivative of the layer below (its output > 0)
         if (!rc && t[5])
             rc = eemd_sg_conv(ptr(t[0]), ptr(t[4]), nullptr, ptr(t[5]), B, T, rows, c, dil, -1, 0, ptr(t[1]),

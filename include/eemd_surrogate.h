@@ -76,8 +76,10 @@ int32_t eemd_sg_pack_layers(const int64_t* table, int32_t n_layers, void* stream
  *            addresses; dx = 0: no input gradient), n_rows, c, nv, cv, dil:
  *            eemd_sg_wgrad, then eemd_sg_conv of dy (dir -1, mask x) into dx.
  * tensor_cores as eemd_sg_conv takes it (in the backward pass the weight
- * gradient runs on the tensor cores when it is not 0).  A refused layer ends
- * the call with its status; the layers before it have been launched. */
+ * gradient runs on the tensor cores when it is not 0).  Every kernel of a pass,
+ * the weight gradients' among them, reports a wait that gave up in *err (may be
+ * null).  A refused layer ends the call with its status; the layers before it
+ * have been launched. */
 int32_t eemd_sg_forward_layers(const int64_t* table, int32_t n_layers, int32_t B, int32_t T, int32_t tensor_cores,
                                int32_t* err, void* stream);
 int32_t eemd_sg_backward_layers(const int64_t* table, int32_t n_layers, int32_t B, int32_t T, int32_t tensor_cores,
