@@ -293,6 +293,12 @@ __device__ __forceinline__ bool wait_parity(uint64_t* bar, uint32_t phase, long 
     return true;
 }
 
+// Polls of the waits that precede a CTA's end: its copies in flight write its
+// shared memory, and its MMAs the tensor memory it frees, until they are done,
+// whether a role gave up or not.  Both end by themselves, so the bound is the
+// default one and not the caller's, which may be short.
+constexpr long long DRAIN_SPINS = 1LL << 24;
+
 // columns [c0, c0 + NC) of this warp's 32 accumulator lanes (NC a multiple of 8)
 template <int NC>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, float (&v)[NC]) {
@@ -835,7 +841,8 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant
             }
             // copies still in flight (only when a role gave up) land before the CTA leaves
             k = max(k, min(nk, NS));
-            for (int j = k - 1; j >= 0 && j >= k - NS; --j) wait_parity(&full[j % NS], (uint32_t)(j / NS) & 1u, spin_limit);
+            for (int j = k - 1; j >= 0 && j >= k - NS; --j)
+                wait_parity(&full[j % NS], (uint32_t)(j / NS) & 1u, DRAIN_SPINS);
         }
     } else if (warp == WS_EPI + 1) {
         // ---------------- MMA warp ----------------
@@ -869,7 +876,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_conv_ws(const __grid_constant
                              : "memory");
             }
             // the issued MMAs are complete before the tensor memory is freed
-            if (k > 0) wait_parity(&accf[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u, spin_limit);
+            if (k > 0) wait_parity(&accf[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u, DRAIN_SPINS);
         }
     } else {
         // ---------------- epilogue warps ----------------
@@ -1373,7 +1380,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constan
             }
             // copies still in flight (only when a role gave up) land before the CTA leaves
             k = max(k, min(nk, NS));
-            for (int j = k - 1; j >= 0 && j >= k - NS; --j) wait_parity(&full[j % NS], (uint32_t)(j / NS) & 1u, spin_limit);
+            for (int j = k - 1; j >= 0 && j >= k - NS; --j)
+                wait_parity(&full[j % NS], (uint32_t)(j / NS) & 1u, DRAIN_SPINS);
         }
     } else if (warp == WG_SUM + 1) {
         // ---------------- MMA warp ----------------
@@ -1408,7 +1416,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constan
                              smem_u32(&accf))
                          : "memory");
             // the issued MMAs are complete before the tensor memory is freed
-            wait_parity(&accf, 0u, spin_limit);
+            wait_parity(&accf, 0u, DRAIN_SPINS);
         }
     } else {
         // ---------------- summing warps ----------------
