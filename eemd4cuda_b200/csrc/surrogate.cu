@@ -1429,7 +1429,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constan
         bool ok = true;
         for (int k = 0; k < nk && ok; ++k) {
             const int s = k % NS;
-            ok = __all_sync(0xffffffffu, wait_parity(&full[s], (uint32_t)(k / NS) & 1u, spin_limit)) && !abort_flag;
+            // (the flag is read inside the vote: another warp may set it between two lanes' reads)
+            ok = __all_sync(0xffffffffu, wait_parity(&full[s], (uint32_t)(k / NS) & 1u, spin_limit) && !abort_flag);
             if (!ok) break;
             const unsigned char* y = sm + s * G::STAGE + 3 * G::XB;
 #pragma unroll
@@ -1443,7 +1444,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_ws(const __grid_constan
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);
         }
-        ok = __all_sync(0xffffffffu, ok && wait_parity(&accf, 0u, spin_limit)) && !abort_flag;
+        ok = __all_sync(0xffffffffu, ok && wait_parity(&accf, 0u, spin_limit) && !abort_flag);
         if (!ok) {
             if (lane == 0) raise(err, EEMD_SG_E_TIMEOUT);
             abort_flag = 1;

@@ -22,3 +22,18 @@ def test_last_waits_do_not_take_the_callers_limit(name):
     unread = re.findall(r"(?:^|[;{})])\s*(wait_parity\([^;]*\));", body(name), flags=re.M)
     assert len(unread) == 2
     assert all(w.endswith("DRAIN_SPINS)") for w in unread), unread
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_a_warps_lanes_agree_on_giving_up(name):
+    """What a vote decides is the same in every lane of a warp only if no lane
+    adds a read of the shared flag after it."""
+    votes = re.findall(r"=\s*(__all_sync\(.*?\));", body(name), flags=re.S)
+    assert votes
+    for v in votes:
+        depth = 0
+        for i, ch in enumerate(v):
+            depth += (ch == "(") - (ch == ")")
+            if depth == 0 and i >= len("__all_sync"):
+                assert v[i + 1:].strip() == "", v
+                break
