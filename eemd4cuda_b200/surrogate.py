@@ -210,10 +210,13 @@ class Net:
     def backward(self, acts, dout, B, T, tensor_cores=True):
         """Gradients of every layer from dL/d(output) (the loss kernel's dout)."""
         self.grads.zero_()
+        # two input-gradient buffers in turn: a layer's is last read by the kernels of the layer
+        # below, before the one after that writes it again
+        bufs = [self.torch.empty((B, T, HIDDEN), dtype=self.torch.bfloat16, device="cuda") for _ in range(2)]
         g, rows = dout, []
         for li in range(len(self.layers) - 1, -1, -1):
             lay = self.layers[li]
-            gi = self.torch.empty((B, T, lay["cin_p"]), dtype=self.torch.bfloat16, device="cuda") if li > 0 else None
+            gi = bufs[li & 1] if li > 0 else None
             rows.append((g, acts[li], lay["dw"], lay["db"], lay["wt"], gi, lay["cout_p"], lay["cin_p"], lay["cout_v"],
                          lay["cin_v"], lay["dil"]))
             g = gi

@@ -1,0 +1,28 @@
+"""Device and host memory that calls and their results hold."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+from eemd4cuda_b200 import surrogate  # noqa: E402
+
+
+def test_backward_holds_two_input_gradients():
+    """Whatever the number of layers: the gradient a layer reads and the one it
+    writes, each [B][T][HIDDEN] in bf16."""
+    B, T = 8, 8192
+    net = surrogate.Net(seed=0)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    inp = torch.randn((B, T, surrogate.CH), generator=g, device="cuda").bfloat16()
+    dout = torch.randn((B, T, surrogate.CH), generator=g, device="cuda").bfloat16()
+    acts = net.forward(inp, B, T)
+    net.backward(acts, dout, B, T)
+    torch.cuda.synchronize()
+    base = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    net.backward(acts, dout, B, T)
+    torch.cuda.synchronize()
+    net.check()
+    one = B * T * surrogate.HIDDEN * 2
+    assert torch.cuda.max_memory_allocated() - base <= 2 * one + (1 << 20)
