@@ -449,7 +449,7 @@ def _run_single(x, *, tau, max_sifts, max_imf, min_extrema, end, rules, exact, d
     xd = torch.from_numpy(np.ascontiguousarray(x, dtype=dt)).to(dev)
     ws = torch.empty((L.workspace_size(p, [N], 1, True),), dtype=torch.uint8, device=dev)
     # (the engine writes every IMF row it returns; the rows past the mode count are not read)
-    # the IMF rows and, behind them, the residual: one copy back
+    # the IMF rows and, behind them, the residual
     rows = torch.empty((slots + 1, N), dtype=tdt, device=dev)
     # the counters in one array (sifts, modes, flags, sifts per mode): one copy back
     cnt = torch.empty((3 + slots,), dtype=torch.int32, device=dev)
@@ -457,14 +457,18 @@ def _run_single(x, *, tau, max_sifts, max_imf, min_extrema, end, rules, exact, d
     L.run(p, xd, [N], 0, 1, ws, imfs=rows, resid_out=rows[slots], nsift=cnt[0:1], nmode=cnt[1:2],
           mode_sifts=cnt[3:], flags=cnt[2:3])
     # every output into pinned memory, one synchronisation
-    h_rows, h_cnt = _pinned(torch, (slots + 1, N), torch.float64), _pinned(torch, (3 + slots,), torch.int32)
-    h_rows.copy_(rows.to(torch.float64), non_blocking=True)
+    # (the residual in memory of its own: a result that keeps only it keeps no IMF rows)
+    h_imfs, h_res = _pinned(torch, (slots, N), torch.float64), _pinned(torch, (N,), torch.float64)
+    h_cnt = _pinned(torch, (3 + slots,), torch.int32)
+    rows = rows.to(torch.float64)
+    h_imfs.copy_(rows[:slots], non_blocking=True)
+    h_res.copy_(rows[slots], non_blocking=True)
     h_cnt.copy_(cnt, non_blocking=True)
     torch.cuda.current_stream(dev).synchronize()
     c = h_cnt.tolist()
     nm = int(c[1])
-    out = h_rows[:nm].numpy()
-    res = h_rows[slots].numpy()
+    out = h_imfs[:nm].numpy()
+    res = h_res.numpy()
     stats = dict(method="gpu", backend="b200", E=1, n_modes=nm, total_sifts=int(c[0]),
                  per_mode_sifts=[int(v) for v in c[3:3 + nm]], per_trial_total_sifts=np.array([int(c[0])]),
                  max_imf_reached=bool(int(c[2]) & 1 and max_imf == -1),

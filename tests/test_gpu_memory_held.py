@@ -5,7 +5,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-from eemd4cuda_b200 import surrogate  # noqa: E402
+from eemd4cuda_b200 import emd_par, surrogate  # noqa: E402
 
 
 def test_backward_holds_two_input_gradients():
@@ -26,3 +26,12 @@ def test_backward_holds_two_input_gradients():
     net.check()
     one = B * T * surrogate.HIDDEN * 2
     assert torch.cuda.max_memory_allocated() - base <= 2 * one + (1 << 20)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_a_kept_residual_keeps_no_imf_rows(dtype):
+    x = np.random.default_rng(2).standard_normal(4096)
+    r = emd_par.decompose(x, E=1, max_imf=5, dtype=dtype)
+    assert r.residual.base.untyped_storage().nbytes() == r.residual.nbytes
+    tol = 1e-12 if dtype is np.float64 else 1e-5  # rounding of the stored rows
+    assert np.max(np.abs(r.imfs.sum(axis=0) + r.residual - x)) <= tol * np.max(np.abs(x))
