@@ -418,8 +418,12 @@ def _run_ensemble(x, *, E, eps, tau, max_sifts, max_imf, min_extrema, end, seed,
         with nvtx.range("eemd.download"):
             n_modes = int(n_modes_d.item())
             ch = cnt.cpu()
-            imfs, residual = mh_host[:n_modes], rh_host
-            _staged_copies(torch, ((imfs, imf_mean[:n_modes]), (residual, resid)), paged)
+            for f in paged:
+                f.result()
+            # the rows past the mode count go back to the system (nothing reads them any more)
+            mh_host.resize((n_modes, N), refcheck=False)
+            imfs, residual = mh_host, rh_host
+            _staged_copies(torch, ((imfs, imf_mean[:n_modes]), (residual, resid)))
     per_trial_sifts, per_trial_modes, flags_all = ch[0].tolist(), ch[1].tolist(), ch[2].tolist()
     if ck is not None:
         ck.remove()

@@ -35,3 +35,14 @@ def test_a_kept_residual_keeps_no_imf_rows(dtype):
     assert r.residual.base.untyped_storage().nbytes() == r.residual.nbytes
     tol = 1e-12 if dtype is np.float64 else 1e-5  # rounding of the stored rows
     assert np.max(np.abs(r.imfs.sum(axis=0) + r.residual - x)) <= tol * np.max(np.abs(x))
+
+
+@pytest.mark.parametrize("max_imf", [-1, 12])
+def test_a_large_ensemble_keeps_its_modes_only(max_imf):
+    """More than 64 MB of IMF slots: the rows past the mode count are given back."""
+    n = 1 << 20
+    x = np.sin(0.05 * np.arange(n))
+    r = emd_par.decompose(x, E=2, eps=1e-3, max_imf=max_imf, seed=1, max_sifts=5)
+    assert r.imfs.shape == (r.n_modes, n) and r.n_modes > 0
+    assert r.imfs.base is None and r.imfs.flags.owndata and r.imfs.flags.writeable
+    assert np.max(np.abs(r.imfs.sum(axis=0) + r.residual - x)) <= 1e-12
