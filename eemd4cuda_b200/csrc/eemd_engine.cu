@@ -282,7 +282,6 @@ template <typename T>
 struct Geo {
     static constexpr int RUN = sizeof(T) == 4 ? 8 : 4;  // consecutive samples per lane
     static constexpr int WT = 32 * RUN;                 // samples per warp tile
-    static constexpr int RS = sizeof(T) == 4 ? 8 : 6;   // workspace elements per interval record
 };
 
 __host__ __device__ inline int stage_pad(int k) { return k + (k >> 4); }
@@ -2062,14 +2061,15 @@ int make_layout(const eemd_params* p, const int64_t* lengths, int n_signals, int
     if (p->reserved > 0 && p->reserved < L.segcap) L.segcap = p->reserved;
 #endif
     L.kcap = (int)(nmax / 2 + 4);
-    const int rs = (p->dtype == EEMD_F64) ? Geo<double>::RS : Geo<float>::RS;
     L.slot_n = pad ? (nmax + row - 1) / row * row : (nmax + 3) / 4 * 4;
     L.slot_runs = (nmax + run - 1) / run + 1;
     L.slots = (int)std::max<int64_t>(
         1, std::min<int64_t>(n_tasks, (int64_t)ASSUMED_SMS * ctas_per_sm(L.nw, p->dtype == EEMD_F64 ? 8 : 4) /
                                      L.csize));
     L.slot_knots = (int64_t)2 * 2 * L.csize * L.nw * L.segcap;
-    L.slot_M = (int64_t)2 * L.kcap * rs;
+    // struct Rec: four coefficients and an index per knot of either envelope, every slot's on 32 bytes
+    const int bm = (p->dtype == EEMD_F64) ? 8 : 4;
+    L.slot_M = ((int64_t)2 * L.kcap * (4 * bm + 4) + 31) / 32 * 32 / bm;
     L.scr_rows = p->exact ? (L.B + L.S) : 0;
     L.NS = ro;
     L.NIMF = imo;
@@ -2095,7 +2095,7 @@ int make_layout(const eemd_params* p, const int64_t* lengths, int n_signals, int
     L.has_w0 = pad && imfs_external && ragged;
     L.o_w0 = take(L.has_w0 ? bt * L.slot_n * L.slots : 0);
     L.o_r1 = take(bt * L.slot_n * L.slots);
-    L.o_ri = take(16 * 2 * L.slot_runs * L.slots);
+    L.o_ri = take(sizeof(uint32_t) * 2 * L.slot_runs * L.slots);
     L.o_scr = take(sizeof(double2) * (size_t)L.scr_rows * L.slots * L.csize * 32 * L.nw);
     L.total = off;
     return EEMD_OK;
