@@ -1892,6 +1892,10 @@ struct Layout {
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// records, and rows where they are padded, are read and written 32 bytes at a
+// time: the arrays lie in the workspace from its first multiple of 32 on
+constexpr size_t WS_ALIGN = 32;
+
 // Clusters of c CTAs of the k_emd instance for (dtype, exact) that the
 // current device can hold at once (0 if the query fails, e.g. no device).
 // the k_emd instance of (storage type, exact, warps per CTA)
@@ -2095,8 +2099,8 @@ int make_layout(const eemd_params* p, const int64_t* lengths, int n_signals, int
     L.has_w0 = pad && imfs_external && ragged;
     L.o_w0 = take(L.has_w0 ? bt * L.slot_n * L.slots : 0);
     L.o_r1 = take(bt * L.slot_n * L.slots);
-    L.o_ri = take(sizeof(uint32_t) * 2 * L.slot_runs * L.slots);
     L.o_scr = take(sizeof(double2) * (size_t)L.scr_rows * L.slots * L.csize * 32 * L.nw);
+    L.o_ri = take(sizeof(uint32_t) * 2 * L.slot_runs * L.slots + WS_ALIGN - 1);  // (the last: what the start skips)
     L.total = off;
     return EEMD_OK;
 }
@@ -2290,7 +2294,7 @@ int32_t eemd_run_traced(const eemd_params* p, const void* x, const int64_t* leng
         if (ws_bytes < L.total) return EEMD_E_NOMEM;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    char* base = static_cast<char*>(ws);
+    char* base = reinterpret_cast<char*>(align_up(reinterpret_cast<uintptr_t>(ws), WS_ALIGN));
     Ctx C;
     memset(&C, 0, sizeof(C));
     C.hdr = reinterpret_cast<Header*>(base + L.o_hdr);

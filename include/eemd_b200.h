@@ -132,7 +132,8 @@ int32_t eemd_philox_normals(uint64_t seed, int32_t signal, int32_t trial_begin, 
  * given lengths (host array) with trial_count trials each.  imfs_external != 0
  * means the caller passes its own per-trial IMF buffer to eemd_run().  The size
  * includes padding that starts every row on 32 bytes; a workspace that holds
- * the rows without it is accepted too and runs them unpadded. */
+ * the rows without it is accepted too and runs them unpadded.  The workspace
+ * may start at any address: what aligning it takes is part of the size. */
 int32_t eemd_workspace_size(const eemd_params* p, const int64_t* lengths,
                             int32_t n_signals, int32_t trial_count,
                             int32_t imfs_external, size_t* ws_bytes);
