@@ -183,6 +183,12 @@ class Net:
         SG.pack_layers([(lay["w"], lay["b"], lay["wp"], lay["wt"], lay["bias"], lay["cout_p"], lay["cin_p"],
                          lay["cout_v"], lay["cin_v"], lay["project"]) for lay in self.layers])
 
+    def layer(self, i, src, dst, B, T, tensor_cores=True):
+        """Layer i alone: dst = layer(src)."""
+        lay = self.layers[i]
+        SG.conv(src, lay["wp"], lay["bias"], dst, B, T, lay["cin_p"], lay["cout_p"], lay["dil"], relu=lay["relu"],
+                tensor_cores=self.conv_kernel if tensor_cores else 0, err=self.err)
+
     def layers_on(self, bufs, B, T, tensor_cores=True):
         """Layer i from bufs[i] to bufs[i + 1], all launched by one call (a call
         and its arguments from Python per layer took longer than a layer of a
