@@ -72,7 +72,11 @@ def launch_shape(n_ref: int, n_tasks: int, dtype: str, n_min: int | None = None,
     1.5 times the samples per CTA slot: the queue hands the longest out first,
     and one that outlasts the rest is the launch's tail (30 signals of 4096 to
     262 144 samples x 32 trials: 66 ms on 1 CTA per task, the median length's
-    entry, 42 on 2, 45 on 3)."""
+    entry, 42 on 2, 45 on 3; of 5 modes x 8 sifts, 50 of 8192 to 131 072 x 8:
+    9.8 ms on 2, the entry, 7.6 on 3, 7.6 on 4; 6 of 16 384 to 1 048 576 x 8:
+    14.6 on 8, 11.3 on 11, 8.4 on 16).  The shortest signal's bound comes
+    first and can cost more than the rule gives: 12 of 2048 to 65 536 x 16 run
+    on 1 in 7.1 ms, where 4 would take 2.3."""
     tab = _table(dtype)
     if not tab:
         return 0, 0

@@ -41,8 +41,11 @@ namespace eemd {
 constexpr int NW_DEFAULT = 4;
 constexpr int MAXNW = 5;
 __host__ __device__ constexpr int ctas_per_sm(int nw, int bt) { return bt == 8 ? 3 : 16 / nw; }
-// largest cluster: portable clusters reach 8 CTAs; 9 to 16 are non-portable
-// and are taken only when the device reports that all of them fit at once
+// largest cluster: portable clusters reach 8 CTAs; 9 to 16 are non-portable.
+// The engine's own rule (cluster_size 0) takes them only when the device reports
+// that all of them fit at once; a size the caller or the table gives is taken as
+// it is (16 CTAs need 4 to 6 SMs of one GPC; a partition of the device with
+// fewer answers EEMD_E_CUDA).
 constexpr int MAXC = 16;
 // owned rows per lane of the fast solve: the forward (c, d) of a pass's rows
 // live in shared memory, so the width costs no registers; odd widths keep the

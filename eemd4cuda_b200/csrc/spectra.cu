@@ -136,7 +136,8 @@ unsigned grid_for(int64_t total) {
 
 // ---------------------------------------------------------------------------
 // Complex FFT of batched rows, this library's own (no FFT library):
-// Stockham autosort passes of radix 4, 2, 3, 5 and of the odd primes up to 31
+// Stockham autosort passes of radix 4, 2, 3, 5 (in shared memory 16 and 8 too)
+// and of the odd primes up to 31
 // (the formulation of Govindaraju et al., "High performance discrete Fourier
 // transforms on graphics processors", SC'08: pass s reads x[j + q N/R],
 // multiplies by the twiddle w^(q k) of the current sub-transform length

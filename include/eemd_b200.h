@@ -90,7 +90,7 @@ typedef struct eemd_params {
     int32_t  tile;            /* samples per warp tile of the fused sift pass: 0, or the only
                                  supported value (256 for float32, 128 for float64) */
     int32_t  knots_per_block; /* owned rows per exact-mode seam window (0 = 16; the fast
-                                 solve owns 3 rows per window) */
+                                 solve owns 5 rows per lane) */
     int32_t  halo;            /* seam halo rows on each side of a window (0 = 32 exact,
                                  24 fast float64, 16 fast float32; at most 64 in fast mode) */
     int64_t  watchdog;        /* >= 0: no effect (the engine has no device waits on its data
@@ -99,7 +99,8 @@ typedef struct eemd_params {
                                  first waits on a flag nothing sets, gives up after k polls
                                  and the run returns EEMD_E_TIMEOUT */
     int32_t  cluster_size;    /* CTAs (thread-block cluster) per task, 1..16 (0 = autotune; 9..16 are
-                                 non-portable cluster sizes the device must support) */
+                                 non-portable sizes, for which one GPC must hold the CTAs:
+                                 EEMD_E_CUDA from the run where it cannot) */
     int32_t  reserved;        /* 0.  Test hook honoured only by the bounds-checked build
                                  (libeemd_b200_checked.so): a value k > 0 caps the knot
                                  lists at k knots of one kind per warp segment, so that

@@ -8,16 +8,18 @@
  *       DC / positive / negative frequencies, inverse FFT), instantaneous
  *       frequency = gradient of the unwrapped phase (np.unwrap, np.gradient
  *       with spacing 1/sr) / 2 pi, instantaneous amplitude = |z|.
- *   eemd_sp_stft        replaces spectra.py:18-29 stft_block:
- *       scipy.signal.stft(window='hann', boundary='zeros', padded=False),
- *       one-sided, divided by the window's sum.
  *       Rows are transformed as real ones (of their own length, or as a circular
  *       convolution with the closed-form Hilbert kernel where the length has a
  *       large prime factor), so neither z nor its spectrum is formed.
+ *   eemd_sp_stft        replaces spectra.py:18-29 stft_block:
+ *       scipy.signal.stft(window='hann', boundary='zeros', padded=False),
+ *       one-sided, divided by the window's sum.
  *   eemd_sp_fft         a complex FFT of any length (numpy.fft.fft's convention
  *       for sign -1, unnormalised), this library's own: Stockham passes of
- *       radix 4, 2, 3, 5 and odd primes up to 31, Bluestein's chirp-z for a
- *       length with a larger prime factor.
+ *       radix 16, 8, 4, 2, 3, 5 and odd primes up to 31 in shared memory (up to
+ *       4096 points, or 4096^2 as two such factors), of radix 4, 2, 3, 5 and
+ *       primes through global memory beyond, Bluestein's chirp-z for a length
+ *       with a larger prime factor.
  *
  * Rows are batched: M signals of N samples each, float64, row-major.  All
  * pointers are device pointers owned by the caller, including the workspace
