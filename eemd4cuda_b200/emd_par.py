@@ -453,25 +453,24 @@ def _run_single(x, *, tau, max_sifts, max_imf, min_extrema, end, rules, exact, d
     xd = torch.from_numpy(np.ascontiguousarray(x, dtype=dt)).to(dev)
     ws = torch.empty((L.workspace_size(p, [N], 1, True),), dtype=torch.uint8, device=dev)
     # (the engine writes every IMF row it returns; the rows past the mode count are not read)
-    # the IMF rows and, behind them, the residual
-    rows = torch.empty((slots + 1, N), dtype=tdt, device=dev)
+    imfs = torch.empty((slots, N), dtype=tdt, device=dev)
+    resid = torch.empty((N,), dtype=tdt, device=dev)
     # the counters in one array (sifts, modes, flags, sifts per mode): one copy back
     cnt = torch.empty((3 + slots,), dtype=torch.int32, device=dev)
     t0 = time.time()
-    L.run(p, xd, [N], 0, 1, ws, imfs=rows, resid_out=rows[slots], nsift=cnt[0:1], nmode=cnt[1:2],
+    L.run(p, xd, [N], 0, 1, ws, imfs=imfs, resid_out=resid, nsift=cnt[0:1], nmode=cnt[1:2],
           mode_sifts=cnt[3:], flags=cnt[2:3])
     # every output into pinned memory, one synchronisation
     # (the residual in memory of its own: a result that keeps only it keeps no IMF rows)
     h_imfs, h_res = _pinned(torch, (slots, N), torch.float64), _pinned(torch, (N,), torch.float64)
     h_cnt = _pinned(torch, (3 + slots,), torch.int32)
-    rows = rows.to(torch.float64)
-    h_imfs.copy_(rows[:slots], non_blocking=True)
-    h_res.copy_(rows[slots], non_blocking=True)
+    h_imfs.copy_(imfs.to(torch.float64), non_blocking=True)
+    h_res.copy_(resid.to(torch.float64), non_blocking=True)
     h_cnt.copy_(cnt, non_blocking=True)
     torch.cuda.current_stream(dev).synchronize()
     c = h_cnt.tolist()
     nm = int(c[1])
-    out = h_imfs[:nm].numpy()
+    out = h_imfs.numpy()[:nm]
     res = h_res.numpy()
     stats = dict(method="gpu", backend="b200", E=1, n_modes=nm, total_sifts=int(c[0]),
                  per_mode_sifts=[int(v) for v in c[3:3 + nm]], per_trial_total_sifts=np.array([int(c[0])]),
