@@ -379,11 +379,11 @@ def measured_peak_hbm():
 # of the same signal and are scaled per (signal, trial) task, since every task
 # streams its own buffers.
 EMD_TRAFFIC = {
-    "harmonic48k": {"bytes_per_launch": 3122266880,
-                    "engine_sha256": "aef4ddc7a17c12bdf012ed251f5fbcd1deabf298ae186f76a95fcb0171e06e9a",
+    "harmonic48k": {"bytes_per_launch": 3110652160,
+                    "engine_sha256": "0819961e765a6766a950b00688c66d7e2ef9bd1b7ac0c59de2de69f766d88d8d",
                     "capture": "one k_emd launch of the 100-trial 48 kHz workload (clusters of 4 five-warp CTAs)"},
-    "amfm4m": {"bytes_per_task": 4268230784.0,
-               "engine_sha256": "aef4ddc7a17c12bdf012ed251f5fbcd1deabf298ae186f76a95fcb0171e06e9a",
+    "amfm4m": {"bytes_per_task": 4264937088.0,
+               "engine_sha256": "0819961e765a6766a950b00688c66d7e2ef9bd1b7ac0c59de2de69f766d88d8d",
                "capture": "one k_emd launch of 4 trials of the 2^22-sample signal (clusters of 16 five-warp "
                           "CTAs), per task"},
 }

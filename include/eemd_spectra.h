@@ -69,7 +69,8 @@ int32_t eemd_sp_stft_shape(int64_t N, int32_t nperseg, int32_t noverlap, int32_t
 /* Workspace bytes for eemd_sp_stft. */
 int32_t eemd_sp_stft_workspace(int32_t M, int64_t N, int32_t nperseg, int32_t noverlap, size_t* bytes);
 
-/* Z[m][f][t] (complex, interleaved re/im float64) of every row x[m][:]. */
+/* Z[m][f][t] (complex, interleaved re/im float64) of every row x[m][:]; x, Z and
+ * the workspace are apart. */
 int32_t eemd_sp_stft(const double* x, int32_t M, int64_t N, int32_t nperseg, int32_t noverlap, double* Z, void* ws,
                      size_t ws_bytes, void* stream);
 
